@@ -126,10 +126,12 @@ int ccp_batch_terms_device(ccp_batch *b, unsigned terms, int nframes, const doub
     if (ncoef < 1 || pgrad_len != 2 * ncoef + 2 * 3 * 289)
       return fail(CCP_ERR_BAD_INPUT, "ccp_batch_terms_device: pgrad_len is not 2 ncoef + 1734");
   }
-  // FS3 of all frames in one launch set when they share one box length
+  // FS3 of all frames in one launch set when they share one box length, and are too narrow for
+  // the pair form, which runs per frame
   bool fused = b->fuse_fs3 && (terms & CCP_TERM_FS3) && nframes > 1 && x && y && z && xs && ys &&
                zs;
   for (int f = 1; fused && f < nframes; f++) fused = box[f] == box[0];
+  if (fused) fused = !ccp::fs3_pair_applies(b->ctx[0], box[0]);
   int model_s3 = 0;
   if (fused) {
     ccp_context_get_option(b->ctx[0], "fs3_available", &model_s3);

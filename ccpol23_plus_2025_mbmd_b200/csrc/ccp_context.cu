@@ -97,6 +97,12 @@ struct ccp_context {
   bool cells_active = false;
   double4 *d_nbrv = nullptr;
   void *d_tri = nullptr;  // FS3 triple records
+  // FS3's pair form (k_fs3_pairs.cu): its lists and tables, allocated by the first evaluation
+  // that uses it
+  Fs3PairBufs fpair{};
+  int fpair_near = 0;      // entries of fpair.near
+  int opt_fs3_pair = 1;    // the pair form where it applies (1) or never (0)
+  bool fs3_pair_active = false;
   int2 *d_pairs = nullptr;
   // reciprocal space
   KVec *d_kv = nullptr;
@@ -227,7 +233,9 @@ void free_ctx(ccp_context *c) {
                 c->d_gfs3,  c->d_vdw_row, c->d_vdw_site, c->d_vdw_qq, c->d_vdw_par,
                 c->d_pcoord, c->d_md_x, c->d_md_xs, c->d_md_v, c->d_md_q, c->d_md_j, c->d_md_red,
                 c->d_mu2, c->d_e0tot, c->d_eim, c->d_T4, c->d_S4, c->d_TB, c->d_SB,
-                c->d_pcg, c->d_cells};
+                c->d_pcg, c->d_cells, c->fpair.near, c->fpair.head, c->fpair.pairv,
+                c->fpair.pairij, c->fpair.vis, c->fpair.vcnt, c->fpair.tab, c->fpair.wtab,
+                c->fpair.vpart};
   for (void *p : dp)
     if (p) cudaFree(p);
   if (c->h_scal) cudaFreeHost(c->h_scal);
@@ -292,6 +300,45 @@ int ensure_lists(ccp_context *c, int cap, int tri_cap, int pair_cap) {
     c->pair_cap = pair_cap;
   }
   return CCP_OK;
+}
+
+// Buffers of FS3's pair form for at least pair_cap pairs and vcap visits per list.  Returns
+// false, with nothing allocated, when the device has no room: the caller then takes the
+// triple form.
+bool ensure_fs3_pairs(ccp_context *c, int pair_cap, int vcap) {
+  Fs3PairBufs &B = c->fpair;
+  const int near = c->nm * c->cap;
+  if (B.tab && pair_cap <= B.pair_cap && vcap <= B.vcap && near <= c->fpair_near) return true;
+  pair_cap = std::max(pair_cap, B.pair_cap);
+  vcap = std::max(vcap, B.vcap);
+  for (void *p : {(void *)B.near, (void *)B.head, (void *)B.pairv, (void *)B.pairij, B.vis,
+                  (void *)B.vcnt, (void *)B.tab, (void *)B.wtab, (void *)B.vpart})
+    if (p) cudaFree(p);
+  B = Fs3PairBufs{};
+  c->fpair_near = 0;
+  const size_t np = pair_cap;
+  char *vis = nullptr;
+  const bool ok = dalloc(&B.near, (size_t)near) == cudaSuccess &&
+                  dalloc(&B.head, (size_t)c->nm) == cudaSuccess &&
+                  dalloc(&B.pairv, np) == cudaSuccess && dalloc(&B.pairij, np) == cudaSuccess &&
+                  dalloc(&vis, np * 2 * vcap * fs3_visit_bytes()) == cudaSuccess &&
+                  dalloc(&B.vcnt, np * 2) == cudaSuccess &&
+                  dalloc(&B.tab, np * 4 * kFs3PairTab) == cudaSuccess &&
+                  dalloc(&B.wtab, np * 2 * kFs3PairTab) == cudaSuccess &&
+                  dalloc(&B.vpart, np * kFs3PairWarps) == cudaSuccess;
+  B.vis = vis;
+  if (!ok) {
+    cudaGetLastError();
+    for (void *p : {(void *)B.near, (void *)B.head, (void *)B.pairv, (void *)B.pairij, B.vis,
+                    (void *)B.vcnt, (void *)B.tab, (void *)B.wtab, (void *)B.vpart})
+      if (p) cudaFree(p);
+    B = Fs3PairBufs{};
+    return false;
+  }
+  B.pair_cap = pair_cap;
+  B.vcap = vcap;
+  c->fpair_near = near;
+  return true;
 }
 
 // Half-space k-vectors with the spherical cut-off, in the reference's loop order
@@ -711,6 +758,20 @@ Fs3Params fs3_params(const ccp_context *c, double box) {
   return F3;
 }
 
+}  // namespace
+
+namespace ccp {
+// The pair form of FS3 serves boxes wider than two FS3 cut-offs: every triple's j-k vector is
+// then the pair's minimum image, so that one table serves all triples of a pair.  It is FP64 in
+// both precision forms: its FP64 sums are faster than the triple form's FP32 passes.
+bool fs3_pair_applies(const ccp_context *c, double box) {
+  const Fs3Params F = fs3_params(c, box);
+  return c->opt_fs3_pair && F.boxb > 2.0 * std::sqrt(F.rc2) * (1.0 + 1e-6);
+}
+}  // namespace ccp
+
+namespace {
+
 // Runs the enabled terms on inputs already in the context's device buffers
 // (x, y, z at px.., sites at pxs.. with leading dimension ld).
 int evaluate_impl(ccp_context *c, const double *px, const double *py, const double *pz,
@@ -775,7 +836,17 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
   // Ewald + induction run on a high-priority internal stream, the three-body terms on
   // low-priority ones, so that freed SM slots go to the latency-bound induction chain first
   cudaStream_t s3 = side ? c->s_fs3 : st, s2 = side ? c->s_fs2 : st, sm = side ? c->s_main : st;
-  for (int attempt = 0; attempt < 3; attempt++) {
+  // FS3 by molecule pairs (k_fs3_pairs.cu) where it applies; otherwise, and without room for
+  // its buffers, by triples
+  bool fs3_pair = (mask & T_FS3) && fs3_pair_applies(c, box);
+  for (int attempt = 0; attempt < 6; attempt++) {
+    if (fs3_pair) {
+      // 17.5 pairs per molecule at the density of liquid water
+      const int pc = c->fpair.pair_cap ? c->fpair.pair_cap : 20 * nm;
+      const int vc = c->fpair.vcap ? c->fpair.vcap : 40;
+      fs3_pair = ensure_fs3_pairs(c, pc, vc);
+    }
+    c->fs3_pair_active = fs3_pair;
     c->launches = 0;
     c->phase_ran = 0;
     pbeg(0, st);
@@ -827,7 +898,18 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       gfs3 = c->d_gfs3;
       CK(cudaMemsetAsync(gfs3, 0, sizeof(double) * kFs3GradLen, s3));
     }
-    if (mask & T_FS3) {
+    if (fs3_pair) {
+      pbeg(7, s3);
+      c->launches++;  // two kernels; LK counts one
+      LK(launch_fs3_pair_lists(c->fpair, c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_s17,
+                               c->d_bgr, c->d_tri, c->tri_cap, c->d_icnt, c->nsm, s3));
+      pend(7, s3);
+      pbeg(8, s3);
+      c->launches++;  // two kernels
+      LK(launch_fs3_pair(c->fpair, c->d_icnt, c->d_comb, c->d_s17, c->d_coef, c->d_bgr, F3, nm, ns,
+                         f3, c->d_fc3, c->d_scal, c->d_tri, c->tri_cap, c->nsm, gfs3, s3));
+      pend(8, s3);
+    } else if (mask & T_FS3) {
       pbeg(7, s3);
       LK(launch_fs3_enum(c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_tri, c->tri_cap,
                          c->d_icnt, s3));
@@ -983,6 +1065,18 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
     if (ic[C_OVERFLOW] > 0) {
       ncap = std::min(nm, ic[C_OVERFLOW] + 32);
       grow = true;
+    }
+    if (fs3_pair) {
+      const int npair = ic[C_NPAIR_FS3], vmax = ic[C_FS3_VMAX];
+      if (ic[C_FS3_MISS] > 0) {
+        fs3_pair = false;
+        grow = true;
+      } else if (npair > c->fpair.pair_cap || vmax > c->fpair.vcap) {
+        const int pc = npair > c->fpair.pair_cap ? npair + npair / 8 + 64 : c->fpair.pair_cap;
+        const int vc = vmax > c->fpair.vcap ? vmax + vmax / 4 + 4 : c->fpair.vcap;
+        fs3_pair = ensure_fs3_pairs(c, pc, vc);
+        grow = true;
+      }
     }
     if (ic[C_NTRI_FS3] > c->tri_cap) {
       ntcap = ic[C_NTRI_FS3] + ic[C_NTRI_FS3] / 4 + 64;
@@ -1552,6 +1646,8 @@ int ccp_context_set_option(ccp_context *ctx, const char *name, int value) {
     ctx->opt_cells = value != 0;
   } else if (n == "pdl") {
     ctx->opt_pdl = value != 0;
+  } else if (n == "fs3_pair_form") {
+    ctx->opt_fs3_pair = value != 0;
   } else if (n == "fs3_fp32_passes") {
     ctx->opt_fs3_low = value != 0;
   } else if (n == "fs3_high_priority") {
@@ -1626,6 +1722,10 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
     *value = ctx->three_body && ctx->s3 && ctx->have_fs3 && ctx->ns >= kNs3 ? 1 : 0;
   } else if (n == "pdl") {
     *value = ctx->opt_pdl;
+  } else if (n == "fs3_pair_form") {
+    *value = ctx->opt_fs3_pair;
+  } else if (n == "fs3_pair_form_active") {
+    *value = ctx->fs3_pair_active ? 1 : 0;
   } else if (n == "fs3_fp32_passes") {
     *value = ctx->opt_fs3_low;
   } else if (n == "fs3_high_priority") {

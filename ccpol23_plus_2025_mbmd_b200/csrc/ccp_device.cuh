@@ -107,6 +107,10 @@ enum CountSlot {
   C_NBLEND_FS3,
   C_NTRI_FS2,
   C_OVERFLOW,
+  C_NPAIR_FS3,  // molecule pairs of FS3's pair form
+  C_FS3_VMAX,   // longest visit list that did not fit
+  C_FS3_MISS,   // triples without one of their pairs
+  C_FS3_TICKET, // triples handed out by the energy kernel after its warps' first
   C_COUNT
 };
 // One more slot past those k_prep clears: set by k_prep when an input coordinate is not
@@ -376,6 +380,33 @@ cudaError_t launch_fs3(int precision, const void *rec, const int *icnt, int tri_
 // the caller).
 cudaError_t launch_fs3_frame_counts(const void *rec, const int *icnt, int tri_cap, int frame_nm,
                                     int *counts, cudaStream_t st);
+// FS3 by molecule pairs (k_fs3_pairs.cu): buffers of the pair form.  near[nm][cap] holds the
+// neighbours of a molecule within FS3's cut-off, head its (count, count below, first pair);
+// pairv/pairij the pairs' vectors (w: squared length) and molecules; vis[pair][SR, LR][vcap] and
+// vcnt[pair][SR, LR] the visit lists; tab[pair][rows][SR, LR] and wtab[pair][SR, LR] the pairs'
+// tables of kFs3PairTab entries; vpart the virial of each block's four warps.
+struct Fs3PairBufs {
+  int *near;
+  int4 *head;
+  double4 *pairv;
+  int2 *pairij;
+  void *vis;
+  int *vcnt;
+  double2 *tab, *wtab;
+  double *vpart;
+  int pair_cap, vcap;
+};
+size_t fs3_visit_bytes();
+constexpr int kFs3PairTab = 296, kFs3PairWarps = 4;
+// tri: fs3_record_bytes() per triple, as launch_fs3_enum's.
+cudaError_t launch_fs3_pair_lists(const Fs3PairBufs &B, const double4 *comb, const int *nbr,
+                                  const int *ncnt, int cap, int nm, Fs3Params P,
+                                  const double4 *s17, const double *bgr, void *tri, int tri_cap,
+                                  int *icnt, int nsm, cudaStream_t st);
+cudaError_t launch_fs3_pair(const Fs3PairBufs &B, const int *icnt, const double4 *comb,
+                            const double4 *s17, const double *coef, const double *bgr, Fs3Params P,
+                            int nm, int ns, double *f, double *fc3, double *scal, void *tri,
+                            int tri_cap, int nsm, double *gfs3, cudaStream_t st);
 cudaError_t launch_fs2_enum(const double4 *comb, const int *nbr, const int *ncnt, int cap,
                             int nm, Fs2Params P, int2 *pairs, int pair_cap, int *icnt,
                             cudaStream_t st);

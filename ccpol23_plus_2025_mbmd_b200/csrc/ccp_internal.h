@@ -47,6 +47,9 @@ int batch_fs3_finish(ccp_context *c, BatchFs3 &B, int nframes, int ld, ccp_energ
                      double *fxs, double *fys, double *fzs, double *fxfs3, double *fyfs3,
                      double *fzfs3, double *pgrad, int pgrad_len);
 
+// Whether FS3 of a box of this length goes by molecule pairs (then it runs per frame).
+bool fs3_pair_applies(const ccp_context *c, double box);
+
 struct Fs3Table {
   double b[289], g[289], r0[289];  // [is*17 + js]
   std::vector<double> cs;          // linear coefficients in file order
