@@ -100,6 +100,7 @@ struct ccp_context {
   // FS3's pair form (k_fs3_pairs.cu): its lists and tables, allocated by the first evaluation
   // that uses it
   Fs3PairBufs fpair{};
+  void *d_fpair = nullptr;  // the one allocation they share
   int fpair_near = 0;      // entries of fpair.near
   int opt_fs3_pair = 1;    // the pair form where it applies (1) or never (0)
   bool fs3_pair_active = false;
@@ -112,7 +113,7 @@ struct ccp_context {
   // row form of the dipole step
   KRow *d_rows = nullptr;
   double *d_rn = nullptr;
-  int nrow = 0, nrow_cap = 0, nrn_cap = 0, row_span = 0;
+  int nrow = 0, nrow_cap = 0, nrn_cap = 0;
   double kv_box = -1, kv_alpha = -1;
   int kv_kmax[3] = {-1, -1, -1};
   double2 *d_tab = nullptr;
@@ -181,7 +182,7 @@ struct ccp_context {
   double2 *d_PM = nullptr;
   size_t PM_cap = 0;
   bool use_PM = false;
-  int opt_pm = 1;  // the full phase matrix when it fits (1) or never (0)
+  int opt_pm = 0;  // the full phase matrix when it fits (1) or never (0)
   // without the full phase matrix, the row form of the dipole step (1) or the factor-table
   // kernels (0)
   int opt_rows = 1;
@@ -233,9 +234,7 @@ void free_ctx(ccp_context *c) {
                 c->d_gfs3,  c->d_vdw_row, c->d_vdw_site, c->d_vdw_qq, c->d_vdw_par,
                 c->d_pcoord, c->d_md_x, c->d_md_xs, c->d_md_v, c->d_md_q, c->d_md_j, c->d_md_red,
                 c->d_mu2, c->d_e0tot, c->d_eim, c->d_T4, c->d_S4, c->d_TB, c->d_SB,
-                c->d_pcg, c->d_cells, c->fpair.near, c->fpair.head, c->fpair.pairv,
-                c->fpair.pairij, c->fpair.vis, c->fpair.vcnt, c->fpair.tab, c->fpair.wtab,
-                c->fpair.vpart};
+                c->d_pcg, c->d_cells, c->d_fpair};
   for (void *p : dp)
     if (p) cudaFree(p);
   if (c->h_scal) cudaFreeHost(c->h_scal);
@@ -302,39 +301,49 @@ int ensure_lists(ccp_context *c, int cap, int tri_cap, int pair_cap) {
   return CCP_OK;
 }
 
-// Buffers of FS3's pair form for at least pair_cap pairs and vcap visits per list.  Returns
-// false, with nothing allocated, when the device has no room: the caller then takes the
-// triple form.
+// Buffers of FS3's pair form for at least pair_cap pairs and vcap visits per list, in one
+// allocation: a cudaMalloc costs 0.4 ms whatever its size, and a context's first evaluation
+// pays for it.  Returns false, with nothing allocated, when the device has no room: the caller
+// then takes the triple form.
 bool ensure_fs3_pairs(ccp_context *c, int pair_cap, int vcap) {
   Fs3PairBufs &B = c->fpair;
   const int near = c->nm * c->cap;
   if (B.tab && pair_cap <= B.pair_cap && vcap <= B.vcap && near <= c->fpair_near) return true;
   pair_cap = std::max(pair_cap, B.pair_cap);
   vcap = std::max(vcap, B.vcap);
-  for (void *p : {(void *)B.near, (void *)B.head, (void *)B.pairv, (void *)B.pairij, B.vis,
-                  (void *)B.vcnt, (void *)B.tab, (void *)B.wtab, (void *)B.vpart})
-    if (p) cudaFree(p);
+  if (c->d_fpair) cudaFree(c->d_fpair);
+  c->d_fpair = nullptr;
   B = Fs3PairBufs{};
   c->fpair_near = 0;
   const size_t np = pair_cap;
-  char *vis = nullptr;
-  const bool ok = dalloc(&B.near, (size_t)near) == cudaSuccess &&
-                  dalloc(&B.head, (size_t)c->nm) == cudaSuccess &&
-                  dalloc(&B.pairv, np) == cudaSuccess && dalloc(&B.pairij, np) == cudaSuccess &&
-                  dalloc(&vis, np * 2 * vcap * fs3_visit_bytes()) == cudaSuccess &&
-                  dalloc(&B.vcnt, np * 2) == cudaSuccess &&
-                  dalloc(&B.tab, np * 4 * kFs3PairTab) == cudaSuccess &&
-                  dalloc(&B.wtab, np * 2 * kFs3PairTab) == cudaSuccess &&
-                  dalloc(&B.vpart, np * kFs3PairWarps) == cudaSuccess;
-  B.vis = vis;
-  if (!ok) {
+  size_t size = 0;
+  auto place = [&](size_t bytes) {  // offset of the next buffer, on a 256-byte boundary
+    const size_t at = size;
+    size = (size + bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t tab = place(np * 4 * kFs3PairTab * sizeof(double2)),
+               wtab = place(np * 2 * kFs3PairTab * sizeof(double2)),
+               vis = place(np * 2 * vcap * fs3_visit_bytes()), pairv = place(np * sizeof(double4)),
+               pairij = place(np * sizeof(int2)), vcnt = place(np * 2 * sizeof(int)),
+               vpart = place(np * kFs3PairWarps * sizeof(double)),
+               nearb = place((size_t)near * sizeof(int)),
+               head = place((size_t)c->nm * sizeof(int4));
+  char *p = nullptr;
+  if (dalloc(&p, size) != cudaSuccess) {
     cudaGetLastError();
-    for (void *p : {(void *)B.near, (void *)B.head, (void *)B.pairv, (void *)B.pairij, B.vis,
-                    (void *)B.vcnt, (void *)B.tab, (void *)B.wtab, (void *)B.vpart})
-      if (p) cudaFree(p);
-    B = Fs3PairBufs{};
     return false;
   }
+  c->d_fpair = p;
+  B.tab = reinterpret_cast<double2 *>(p + tab);
+  B.wtab = reinterpret_cast<double2 *>(p + wtab);
+  B.vis = p + vis;
+  B.pairv = reinterpret_cast<double4 *>(p + pairv);
+  B.pairij = reinterpret_cast<int2 *>(p + pairij);
+  B.vcnt = reinterpret_cast<int *>(p + vcnt);
+  B.vpart = reinterpret_cast<double *>(p + vpart);
+  B.near = reinterpret_cast<int *>(p + nearb);
+  B.head = reinterpret_cast<int4 *>(p + head);
   B.pair_cap = pair_cap;
   B.vcap = vcap;
   c->fpair_near = near;
@@ -427,15 +436,6 @@ int ensure_kspace(ccp_context *c, double box) {
   {
     std::vector<KRow> rows = build_krows(kv, c->kmax[1]);
     c->nrow = (int)rows.size();
-    c->row_span = 0;
-    for (int t = 0; t < c->nrow; t += kRowTile) {
-      int nb = rows[t].nlo, ne = nb + rows[t].len;
-      for (int r = t + 1; r < std::min(c->nrow, t + kRowTile); r++) {
-        nb = std::min(nb, rows[r].nlo);
-        ne = std::max(ne, rows[r].nlo + rows[r].len);
-      }
-      c->row_span = std::max(c->row_span, ne - nb);
-    }
     if (c->nrow > c->nrow_cap) {
       if (c->d_rows) cudaFree(c->d_rows);
       c->d_rows = nullptr;
@@ -494,9 +494,8 @@ struct EvalOut {
 // polarisable site: 5 MB at 512 waters, 46 MB at 2048).
 constexpr size_t kPhaseBudget = size_t(1) << 30;
 // The full phase matrix (16 bytes per polarisable site and k-vector: 38 MB at 512 waters,
-// 568 MB at 2048) pays only while it stays in L2, which it is read from twice per step: it
-// is used when it fits in half of the L2.  Streamed from HBM (2048 waters) it made the dipole
-// step slower than the factor tables and evicted the concurrent kernels' working sets.
+// 568 MB at 2048), an option, is used when it fits in half of the L2, which it is read from
+// twice per step.
 size_t full_phase_budget(const ccp_context *c) { return c->l2_bytes / 2; }
 
 constexpr double kIndThr = 1.0e-20;  // iteridm convergence threshold on sum |dmu|^2
@@ -544,10 +543,10 @@ IterArgs make_iter_args(ccp_context *c, cudaGraphConditionalHandle handle, int u
     A.XY = nullptr;
     A.rows = c->d_rows;
     A.nrow = c->nrow;
-    A.row_span = c->row_span;
+    A.row_sites = iter_row_sites(A.nw, c->nrow);
+    A.zs = 8 * iter_row_tiles(c->kmax[2]);
     A.XYr = c->d_P;
-    A.Z = c->d_P + (size_t)c->nrow * A.nw;
-    A.ZT = A.Z + (size_t)A.nz * A.nw;
+    A.Zc = reinterpret_cast<const double *>(c->d_P + (size_t)((c->nrow + 7) / 8 * 8) * A.nw);
     A.rn = c->d_rn;
   }
   A.sk = c->d_skj;
@@ -615,7 +614,7 @@ int ensure_ind_graph(ccp_context *c) {
       (long long)c->use_P, (long long)c->d_PM, (long long)c->use_PM, c->cap, c->nm, c->nk, c->kmax[0], c->kmax[1], c->kmax[2], c->maxit,
       (long long)pcg_solver(c), (long long)c->opt_solver, (long long)c->d_pcg,
       (long long)c->opt_pdl, c->opt_sum_sites, c->opt_gather_sites, (long long)c->use_rows,
-      (long long)c->d_rows, c->nrow, c->row_span, (long long)c->d_rn};
+      (long long)c->d_rows, c->nrow, (long long)c->d_rn};
   double thr = ind_threshold(c);
   long long thr_bits;
   std::memcpy(&thr_bits, &thr, sizeof thr_bits);
@@ -711,16 +710,15 @@ int run_dipole_loop(ccp_context *c, cudaStream_t st) {
 // Allocates the phase-factor tables when the dipole iteration can use them.
 int ensure_phase_matrix(ccp_context *c) {
   const size_t nw = (size_t)c->nm * c->S.np, nz = 2 * (size_t)c->kmax[2] + 1;
-  // XY[site][l][m] and Z[site][n], or in the row form XYr[row][site], Z and ZT[n][site]
+  // XY[site][l][m] and Z[site][n], or in the row form XYt[row tile][site][row] and Zc[site][n]
   const size_t n = nw * std::max((size_t)(c->kmax[0] + 1) * (2 * c->kmax[1] + 1) + nz,
-                                 (size_t)c->nrow + 2 * nz);
+                                 (size_t)(c->nrow + 7) / 8 * 8 + 4 * iter_row_tiles(c->kmax[2]));
   // the gather records pack the phase-table row of n in 8 bits
   c->use_P = c->opt_phase && c->nk > 0 && n * sizeof(double2) <= kPhaseBudget &&
              2 * c->kmax[2] + 1 <= 255;
   const size_t npm = (size_t)c->nm * c->S.np * (size_t)c->nk;
   c->use_PM = c->use_P && c->opt_pm && npm * sizeof(double2) <= full_phase_budget(c);
-  c->use_rows = c->use_P && !c->use_PM && c->opt_rows &&
-                iter_rows_fit(c->opt_sum_sites, 2 * c->kmax[2] + 1, c->row_span);
+  c->use_rows = c->use_P && !c->use_PM && c->opt_rows && iter_rows_fit(c->kmax[2]);
   if (c->use_P && n > c->P_cap) {
     if (c->d_P) cudaFree(c->d_P);
     c->d_P = nullptr;
@@ -980,10 +978,10 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       LK(launch_kspace_gather(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
                               c->kmax[2], c->d_mu, c->d_sk, c->d_e0k, fk, sk));
       if (c->use_rows) {
-        const size_t nw = (size_t)nm * S.np, nz = 2 * c->kmax[2] + 1;
-        double2 *XYr = c->d_P, *Z = XYr + (size_t)c->nrow * nw, *ZT = Z + nz * nw;
+        double2 *Zc = c->d_P + (size_t)((c->nrow + 7) / 8 * 8) * nm * S.np;
         LK(launch_phase_rows(c->d_tab, nm, S, c->kmax[0], c->kmax[1], c->kmax[2], c->d_rows,
-                             c->nrow, XYr, Z, ZT, sk));
+                             c->nrow, 8 * iter_row_tiles(c->kmax[2]), c->d_P,
+                             reinterpret_cast<double *>(Zc), sk));
       } else if (c->use_P) {
         const int nlm = (c->kmax[0] + 1) * (2 * c->kmax[1] + 1), nz = 2 * c->kmax[2] + 1;
         double2 *XY = c->d_P, *Z = c->d_P + (size_t)nm * S.np * nlm;

@@ -165,7 +165,7 @@ struct KRow {
   double rl, rm;
   int kbeg, len, nlo, lm;
 };
-constexpr int kRowTile = 32;  // rows per structure-factor block of the row form
+constexpr int kRowTilesMax = 5;  // tiles of four n = 0 .. n_max that the row form takes
 
 // Arguments of one step of the dipole solve with the phase matrix (k_iter.cu): a Jacobi step,
 // or with cu.. set a preconditioned-conjugate-gradient step.
@@ -189,12 +189,14 @@ struct IterArgs {
   // from the factor rows
   const double2 *PM;
   // the row form (PM null, rows set): the k-vector rows by decreasing length, the factor
-  // tables XYr[r][w] = exp(i(l x + m y)) of row r and site w, Z[w][n] as above and its
-  // transpose ZT[n][w], and rn[n + nmax] = 2 pi n / L
+  // tables XYr[tile of 8 rows][w][row] = exp(i(l x + m y)) and Zc[w][2 n + {0, 1}] =
+  // (cos, sin)(n z) for n >= 0 (k_phase_rows), and rn[n + nmax] = 2 pi n / L
   const KRow *rows;
   int nrow;
-  int row_span;  // the largest n range of a tile of kRowTile consecutive rows
-  const double2 *XYr, *ZT;
+  int row_sites;  // polarisable sites per structure-factor block
+  int zs;         // doubles per site in Zc
+  const double2 *XYr;
+  const double *Zc;
   const double *rn;
   // sk[k] holds two S(k) buffers, (re, im) of steps of parity 0 and 1: a step accumulates
   // into its own and clears the other, which the previous step's gather has finished with
@@ -317,12 +319,13 @@ cudaError_t launch_phase_factors(const double2 *tab, int nm, SiteSets S, int kl,
 cudaError_t launch_tmu(const int *nbr, const int *ncnt, int cap, int nm, int np, const double4 *T4,
                        const double *TB, const double4 *S4, const double *SB, const double *mu,
                        double *eim, cudaStream_t st);
-size_t iter_rows_smem_a(int sum_sites, int row_span);
-size_t iter_rows_smem_b(int nz, int row_span);
-bool iter_rows_fit(int sum_sites, int nz, int row_span);
+int iter_row_tiles(int nmax);
+bool iter_rows_fit(int nmax);
+int iter_row_sites(int nw, int nrow);
+// zs = 8 iter_row_tiles(kn) doubles per site in Zc.
 cudaError_t launch_phase_rows(const double2 *tab, int nm, SiteSets S, int kl, int km, int kn,
-                              const KRow *rows, int nrow, double2 *XYr, double2 *Z,
-                              double2 *ZT, cudaStream_t st);
+                              const KRow *rows, int nrow, int zs, double2 *XYt, double *Zc,
+                              cudaStream_t st);
 cudaError_t launch_phase_matrix(const KGather *kg, int nk, int nw, int nlm, int nz,
                                 const double2 *XY, const double2 *Z, double2 *PM,
                                 cudaStream_t st);

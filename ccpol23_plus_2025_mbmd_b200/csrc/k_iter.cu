@@ -22,12 +22,10 @@
 //      of a graph body that unrolls several steps then returns at once) and, inside the
 //      graph, sets the WHILE node's condition.  S(k) alternates between two buffers by step
 //      parity, so no block has to clear it after the gather.
-// When the full phase matrix [site][k] fits in L2 both passes read one phase per pair from
-// it; otherwise the row form (k_iter_a_rows, k_iter_b_rows below) takes the sums row by row
-// of the k-vector list from factors staged in shared memory.  The same step can also run on
-// the factor tables alone (k_iter_a/k_iter_b without the matrix).
-#include <climits>
-
+// The step normally runs in the row form (k_iter_a_rows, k_iter_b_rows below), which takes the
+// reciprocal sums as matrix products over the rows of the k-vector list.  k_iter_a and k_iter_b
+// take them k-vector by k-vector, from the factor tables (k_max above the row form's) or, by
+// option, from the full phase matrix [site][k].
 #include "ccp_device.cuh"
 
 using namespace ccpd;
@@ -91,45 +89,40 @@ __global__ void k_phase_factors(const double2 *__restrict__ tab, int nm, SiteSet
   }
 }
 
-// The factor tables of the row form: XYr[r][w] for the k-vector rows (KRow, lm = l (2 mmax +
-// 1) + m + mmax), formed as k_phase_factors forms XY, and Z both as Z[w][n] and as its
-// transpose ZT[n][w].  Site-fastest order, so the row-major writes and the per-axis table
-// reads coalesce.
+// The factor tables of the row form: XYt[row tile of 8][w][row in tile] = exp(i(l x + m y)) of
+// the k-vector rows (KRow, lm = l (2 mmax + 1) + m + mmax), formed as k_phase_factors forms XY,
+// zero past the last row; and Zc[w][2 n + {0, 1}] = (cos, sin)(n z), n = 0 .. zs / 2 - 1, zero
+// past nmax.  A tile's rows are the fastest index, so that an operand fragment of 8 rows x 4
+// sites is 512 contiguous bytes.
 __global__ void k_phase_rows(const double2 *__restrict__ tab, int nm, SiteSets S, int k1,
-                             int mmax, int nmax, const KRow *__restrict__ rows, int nrow,
-                             double2 *XYr, double2 *Z, double2 *ZT) {
+                             int mmax, int nmax, const KRow *__restrict__ rows, int nrow, int zs,
+                             double2 *XYt, double2 *Zc) {
   const int nw = nm * S.np;
-  const int M = 2 * mmax + 1, nz = 2 * nmax + 1;
+  const int M = 2 * mmax + 1, nt8 = (nrow + 7) / 8;
   const size_t N = (size_t)nm * S.na;
-  const size_t nxy = (size_t)nrow * nw, total = nxy + (size_t)nz * nw;
+  const size_t nxy = (size_t)nt8 * nw * 8, total = nxy + (size_t)nw * (zs / 2);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
        t += (size_t)gridDim.x * blockDim.x) {
     if (t < nxy) {
-      const int r = (int)(t / nw), w = (int)(t - (size_t)r * nw);
-      const int i = w / S.np, p = w % S.np;
-      const size_t st = (size_t)i * S.na + S.a_of_p[p];
-      const int lm = rows[r].lm, l = lm / M, m = lm % M - mmax;
-      const double2 el = tab[(size_t)(0 * k1 + l) * N + st];
-      const double2 em = tab[(size_t)(1 * k1 + (m < 0 ? -m : m)) * N + st];
-      double clm, slm;
-      if (m >= 0) {
-        clm = el.x * em.x - el.y * em.y;
-        slm = el.y * em.x + em.y * el.x;
-      } else {
-        clm = el.x * em.x + el.y * em.y;
-        slm = el.y * em.x - em.y * el.x;
+      const size_t u = t >> 3;
+      const int rt = (int)(u / nw), w = (int)(u - (size_t)rt * nw), r = rt * 8 + (int)(t & 7);
+      double2 xy = make_double2(0.0, 0.0);
+      if (r < nrow) {
+        const int i = w / S.np, p = w % S.np;
+        const size_t st = (size_t)i * S.na + S.a_of_p[p];
+        const int lm = rows[r].lm, l = lm / M, m = lm % M - mmax;
+        const double2 el = tab[(size_t)(0 * k1 + l) * N + st];
+        const double2 em = tab[(size_t)(1 * k1 + (m < 0 ? -m : m)) * N + st];
+        xy = m >= 0 ? make_double2(el.x * em.x - el.y * em.y, el.y * em.x + em.y * el.x)
+                    : make_double2(el.x * em.x + el.y * em.y, el.y * em.x - em.y * el.x);
       }
-      XYr[t] = make_double2(clm, slm);
+      XYt[t] = xy;
     } else {
       const size_t u = t - nxy;
-      const int ni = (int)(u / nw), w = (int)(u - (size_t)ni * nw);
+      const int w = (int)(u / (zs / 2)), n = (int)(u - (size_t)w * (zs / 2));
       const int i = w / S.np, p = w % S.np;
       const size_t st = (size_t)i * S.na + S.a_of_p[p];
-      const int n = ni - nmax;
-      const double2 en = tab[(size_t)(2 * k1 + (n < 0 ? -n : n)) * N + st];
-      const double2 z = make_double2(en.x, n < 0 ? -en.y : en.y);
-      ZT[u] = z;
-      Z[(size_t)w * nz + ni] = z;
+      Zc[u] = n <= nmax ? tab[(size_t)(2 * k1 + n) * N + st] : make_double2(0.0, 0.0);
     }
   }
 }
@@ -559,46 +552,43 @@ __global__ void __launch_bounds__(kGatherThreads)
 }
 
 // ------------------------------------------------------------------ the row form
-// For boxes whose phase matrix does not fit in L2 the step kernels above form each (site,
-// k-vector) phase from two factor-table loads, and both passes then run at the L1 load rate,
-// far below the FP64 rate.  The row form regroups the same sums by the rows of the k-vector
-// list (one (l, m), a run of n), so that every loaded value serves many products:
+// The step's two reciprocal sums regrouped by the rows of the k-vector list (one (l, m), a run
+// of n), which makes them small matrix products for the FP64 tensor cores:
 //   structure factors  S(k) = sum_w Z(w, n) (B(w, r) + k_n C(w, r)),
-//                      B = XY(w, r) (k_l mu_x + k_m mu_y),  C = XY(w, r) mu_z;
+//                      B = XY(w, r) (k_l mu_x + k_m mu_y),  C = XY(w, r) mu_z:
+//     the real and imaginary parts of B and C (8 rows x sites) times (cos, sin)(n z) (sites x n
+//     >= 0); +n and -n come from the same four real sums;
 //   gather             E(w) = sum_r Re[XY(w, r) (k_l Q, k_m Q, Q_z)],
-//                      Q = sum_n Z(w, n) conj F(k),  Q_z = sum_n k_n Z(w, n) conj F(k),
-// F(k) the weighted S(k) of the step.  These are k_iter_a's and k_iter_b's sums with the
-// products reassociated (equal to rounding).
-constexpr int kRowLanes = 8;  // n lanes per row of a structure-factor block: n = nb + lane + 8 j
-// gather blocks: sites per block (8, 16 or 32), rows per thread, warps per block
-#ifndef CCP_ROW_SITES
-#define CCP_ROW_SITES 16
-#endif
-#ifndef CCP_ROW_R
-#define CCP_ROW_R 4
-#endif
-#ifndef CCP_ROW_WARPS
-#define CCP_ROW_WARPS 8
-#endif
-// structure-factor blocks resident per SM that the register allocation targets
-#ifndef CCP_ROW_SUM_BLOCKS
-#define CCP_ROW_SUM_BLOCKS 1
-#endif
-constexpr int kRowSites = CCP_ROW_SITES, kRowR = CCP_ROW_R, kRowWarps = CCP_ROW_WARPS;
-constexpr int kRowSumBlocks = CCP_ROW_SUM_BLOCKS;
-static_assert(kRowSites == 8 || kRowSites == 16 || kRowSites == 32, "sites per gather block");
-static_assert(kThreads / kRowLanes * 2 == kRowTile, "a structure-factor block takes two rows per thread");
+//                      Q = sum_n Z(w, n) conj F(k),  Q_z = sum_n k_n Z(w, n) conj F(k):
+//     (cos, sin)(n z) (8 sites x n) times F's combinations over +-n (n x rows), F(k) the
+//     weighted S(k) of the step.
+// Both read the factor tables once per step (3 MB at 512 waters, where the phase matrix takes
+// 38 MB twice), and XY serves 2 n_max + 1 k-vectors per load.  These are k_iter_a's and
+// k_iter_b's sums with the products reassociated (equal to rounding).
 
-// Structure factors of the row form: block b (after the T.mu blocks) covers tile b % ntile
-// (kRowTile consecutive rows of the length-sorted list, n in [nb, ne) of their union) and the
-// sites of chunk b / ntile.  A thread takes two adjacent rows of the tile and the n = nb +
-// lane + 8 j (j < J) of them, so that each Z factor it loads serves both; the partial sums are
-// merged with FP64 atomics as in k_iter_a.  The chunk's XY factors of the tile's rows and its
-// Z factors of the tile's n range are staged in shared memory before the wait for the
-// previous step (the tables are fixed during the solve), so the site loop reads only shared
-// memory.
+// D = A (8x4) B (4x8) + C in FP64: lane l holds A[l/4][l%4], B[l%4][l/4] and C, D
+// [l/4][2 (l%4) + {0, 1}].
+__device__ __forceinline__ void dmma(double2 &d, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d.x), "+d"(d.y)
+      : "d"(a), "d"(b));
+}
+
+constexpr int kRowSteps = 6;  // steps of four sites whose XY a warp loads before it waits
+constexpr int kRowWarps = 8;  // warps of a gather block, each taking row tiles in turn
+
+// the largest n of the rows of a lane's tile (rows sorted by length: only the row (0, 0), which
+// has no n < 1, can reach further than its neighbours)
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
+// Structure factors: block b (after the T.mu blocks) covers row tile b % nt8 and the sites of
+// chunk b / nt8 (A.row_sites of them), its four warps a quarter each.  A lane forms the four
+// operands (Re, Im of B and C) of its row and site from one XY load; J tiles of four n.  The
+// warps' partial sums meet in shared memory, and one thread per (row, n) combines them into
+// S(r, n) and S(r, -n), merged with FP64 atomics as in k_iter_a.  The first steps' XY are
+// loaded before the wait for the previous step (the tables are fixed during the solve).
 template <bool PCG, int J>
-__global__ void __launch_bounds__(kThreads, kRowSumBlocks) k_iter_a_rows(IterArgs A) {
+__global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
   const int nA = (A.nw + kWarps - 1) / kWarps;
   if ((int)blockIdx.x < nA) {
     pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
@@ -607,228 +597,205 @@ __global__ void __launch_bounds__(kThreads, kRowSumBlocks) k_iter_a_rows(IterArg
     iter_a_tmu<PCG>(A, pin, nA);
     return;
   }
-  // the chunk's dipoles [site] (x, y, z, 0), the XY factors [site][row] of the tile's rows and
-  // the Z factors [site][n - nb] of its n range (row stride row_span)
-  extern __shared__ double4 smu4[];
-  constexpr int kXs = kRowTile + 1;  // site stride of the staged XY: no bank conflicts
-  double2 *bxy = reinterpret_cast<double2 *>(smu4 + A.sum_sites);
-  double2 *zs = bxy + (size_t)A.sum_sites * kXs;
-  __shared__ int s_nb, s_ne;
-  const int b = blockIdx.x - nA;
-  const int ntile = (A.nrow + kRowTile - 1) / kRowTile;
-  const int rt = b % ntile, sc = b / ntile;
-  const int s0 = sc * A.sum_sites, cnt = min(A.sum_sites, A.nw - s0);
-  const int r0 = rt * kRowTile, nr = min(kRowTile, A.nrow - r0);
-  if (threadIdx.x == 0) {
-    int nb = A.rows[r0].nlo, ne = nb + A.rows[r0].len;
-    for (int r = 1; r < nr; r++) {
-      const int lo = A.rows[r0 + r].nlo;
-      nb = min(nb, lo);
-      ne = max(ne, lo + A.rows[r0 + r].len);
-    }
-    s_nb = nb;
-    s_ne = ne;
-  }
-  for (int u = threadIdx.x; u < nr * cnt; u += kThreads) {
-    const int r = u / cnt, s = u - r * cnt;
-    bxy[s * kXs + r] = A.XYr[(size_t)(r0 + r) * A.nw + s0 + s];
-  }
-  __syncthreads();
-  const int nb = s_nb, nn = s_ne - nb;  // nn <= row_span
-  for (int u = threadIdx.x; u < cnt * nn; u += kThreads) {
-    const int s = u / nn, j = u - s * nn;
-    zs[s * A.row_span + j] = A.Z[(size_t)(s0 + s) * A.nz + nb + j + A.nmax];
-  }
+  extern __shared__ double4 smu4[];  // A.row_sites dipoles, then the warps' sums
+  double2(*red)[4 * J][32] = reinterpret_cast<double2(*)[4 * J][32]>(smu4 + A.row_sites);
+  const int b = blockIdx.x - nA, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nt8 = (A.nrow + 7) / 8, rt = b % nt8, s0 = b / nt8 * A.row_sites;
+  const int r = min(rt * 8 + (lane >> 2), A.nrow - 1);
+  const KRow R = A.rows[r];
+  const int jt = warp_max(R.nlo + R.len - 1) / 4 + 1;  // n tiles of the row tile
+  const int q0 = wid * (A.row_sites / 4) + (lane & 3);  // lane's site in the chunk, step 0
+  const int steps = min(A.row_sites / 16, (A.nw - s0 - wid * (A.row_sites / 4) + 3) / 4);
+  const double2 *xyt = A.XYr + (size_t)rt * A.nw * 8 + (lane >> 2);
+  double2 xy[kRowSteps];
+#pragma unroll
+  for (int t = 0; t < kRowSteps; t++)
+    xy[t] = xyt[(size_t)min(s0 + q0 + 4 * t, A.nw - 1) * 8];
   pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
   PcgIn pin;
   if constexpr (PCG) pin = pcg_in(A);
-  for (int u = threadIdx.x; u < cnt; u += kThreads) {
-    const size_t o = (size_t)(s0 + u) * 3;
-    if constexpr (PCG) {
-      const double ap = pin.apol((s0 + u) % A.np);
-      smu4[u] = make_double4(pin.comp(o, ap), pin.comp(o + 1, ap), pin.comp(o + 2, ap), 0.0);
-    } else {
-      smu4[u] = make_double4(A.mu[o], A.mu[o + 1], A.mu[o + 2], 0.0);
-    }
-  }
-  __syncthreads();
-  const int ra = 2 * (threadIdx.x / kRowLanes), c = threadIdx.x % kRowLanes;
-  if (ra >= nr) return;
-  // this thread's rows ra and ra + 1 of the tile (the second empty past the tile's end)
-  const KRow R0 = A.rows[r0 + ra];
-  KRow R1 = R0;
-  if (ra + 1 < nr)
-    R1 = A.rows[r0 + ra + 1];
-  else
-    R1.len = 0;
-  const int rb1 = ra + 1 < nr ? ra + 1 : ra;
-  const int jt = (nn + kRowLanes - 1) / kRowLanes;  // jt <= J: row_span
-  // per n = nb + c + 8 j: the staged Z column (clamped to the range, so idle lanes read a
-  // column another lane reads), k_n, and the k-vector of each row that holds that n
-  int col[J], k0[J], k1[J];
-  double rnj[J];
-#pragma unroll
-  for (int j = 0; j < J; j++) {
-    const int d = c + kRowLanes * j, n = nb + d;
-    col[j] = min(d, nn - 1);
-    rnj[j] = d < nn ? A.rn[n + A.nmax] : 0.0;
-    k0[j] = j < jt && n >= R0.nlo && n < R0.nlo + R0.len ? R0.kbeg + (n - R0.nlo) : -1;
-    k1[j] = j < jt && n >= R1.nlo && n < R1.nlo + R1.len ? R1.kbeg + (n - R1.nlo) : -1;
-  }
-  double ax[J], ay[J], bx_[J], by_[J];
-#pragma unroll
-  for (int j = 0; j < J; j++) ax[j] = ay[j] = bx_[j] = by_[j] = 0.0;
-#pragma unroll 2
-  for (int s = 0; s < cnt; s++) {
-    const double4 m = smu4[s];
-    const double2 xy0 = bxy[s * kXs + ra], xy1 = bxy[s * kXs + rb1];
-    const double a0 = R0.rl * m.x + R0.rm * m.y, a1 = R1.rl * m.x + R1.rm * m.y;
-    const double b0x = xy0.x * a0, b0y = xy0.y * a0, c0x = xy0.x * m.z, c0y = xy0.y * m.z;
-    const double b1x = xy1.x * a1, b1y = xy1.y * a1, c1x = xy1.x * m.z, c1y = xy1.y * m.z;
-    const double2 *zw = zs + s * A.row_span;
-#pragma unroll
-    for (int j = 0; j < J; j++) {
-      if (j < jt) {
-        const double2 z = zw[col[j]];
-        const double t0x = rnj[j] * c0x + b0x, t0y = rnj[j] * c0y + b0y;
-        const double t1x = rnj[j] * c1x + b1x, t1y = rnj[j] * c1y + b1y;
-        ax[j] += z.x * t0x - z.y * t0y;
-        ay[j] += z.x * t0y + z.y * t0x;
-        bx_[j] += z.x * t1x - z.y * t1y;
-        by_[j] += z.x * t1y + z.y * t1x;
+  for (int u = threadIdx.x; u < A.row_sites; u += kThreads) {
+    double4 m = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (s0 + u < A.nw) {
+      const size_t o = (size_t)(s0 + u) * 3;
+      if constexpr (PCG) {
+        const double ap = pin.apol((s0 + u) % A.np);
+        m = make_double4(pin.comp(o, ap), pin.comp(o + 1, ap), pin.comp(o + 2, ap), 0.0);
+      } else {
+        m = make_double4(A.mu[o], A.mu[o + 1], A.mu[o + 2], 0.0);
       }
     }
+    smu4[u] = m;
+  }
+  __syncthreads();
+  double2 acc[4][J];
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int j = 0; j < J; j++) acc[c][j] = make_double2(0.0, 0.0);
+  for (int t0 = 0; t0 < steps; t0 += kRowSteps) {
+#pragma unroll
+    for (int t = 0; t < kRowSteps; t++) {
+      if (t0 + t < steps) {  // warp-uniform
+        const int q = q0 + 4 * (t0 + t), w = min(s0 + q, A.nw - 1);  // mu = 0 past the last site
+        const double *z = A.Zc + (size_t)w * A.zs + (lane >> 2);
+        double zf[J];
+#pragma unroll
+        for (int j = 0; j < J; j++) zf[j] = j < jt ? z[8 * j] : 0.0;
+        const double4 m = smu4[q];
+        const double d = R.rl * m.x + R.rm * m.y;
+        const double a[4] = {xy[t].x * d, xy[t].y * d, xy[t].x * m.z, xy[t].y * m.z};
+#pragma unroll
+        for (int j = 0; j < J; j++)
+          if (j < jt)
+#pragma unroll
+            for (int c = 0; c < 4; c++) dmma(acc[c][j], a[c], zf[j]);
+      }
+    }
+    if (t0 + kRowSteps < steps)
+#pragma unroll
+      for (int t = 0; t < kRowSteps; t++)
+        xy[t] = xyt[(size_t)min(s0 + q0 + 4 * (t0 + kRowSteps + t), A.nw - 1) * 8];
   }
   pdl_launch_dependents();
 #pragma unroll
-  for (int j = 0; j < J; j++) {
-    // kspace_efield_idm's weight (nb_induction_model.f90:2560-2600), applied before the merge
-    if (k0[j] >= 0) {
-      const double g = -4.0 * A.kv[k0[j]].ak;
-      atomicAdd(&A.sk[(size_t)k0[j] * 4 + 2 * A.par], g * ax[j]);
-      atomicAdd(&A.sk[(size_t)k0[j] * 4 + 2 * A.par + 1], g * ay[j]);
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int j = 0; j < J; j++) red[wid][c * J + j][lane] = acc[c][j];
+  __syncthreads();
+  // lane l of a warp's results is row l / 4 and n = 4 j + l % 4: (cos, sin) sums of each part
+  for (int u = threadIdx.x; u < jt * 32; u += kThreads) {
+    const int j = u >> 5, l = u & 31, row = rt * 8 + (l >> 2), n = 4 * j + (l & 3);
+    if (row >= A.nrow || n > A.nmax) continue;
+    double2 v[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      v[c] = red[0][c * J + j][l];
+#pragma unroll
+      for (int w = 1; w < kWarps; w++) {
+        const double2 x = red[w][c * J + j][l];
+        v[c].x += x.x;
+        v[c].y += x.y;
+      }
     }
-    if (k1[j] >= 0) {
-      const double g = -4.0 * A.kv[k1[j]].ak;
-      atomicAdd(&A.sk[(size_t)k1[j] * 4 + 2 * A.par], g * bx_[j]);
-      atomicAdd(&A.sk[(size_t)k1[j] * 4 + 2 * A.par + 1], g * by_[j]);
+    const KRow K = A.rows[row];
+    const double kn = A.rn[n + A.nmax];
+    // B + k_n C (n), B - k_n C (-n), times cos +- i sin
+    const double pr = (v[0].x - v[1].y) + kn * (v[2].x - v[3].y);
+    const double pi = (v[0].y + v[1].x) + kn * (v[2].y + v[3].x);
+    const double mr = (v[0].x + v[1].y) - kn * (v[2].x + v[3].y);
+    const double mi = (v[1].x - v[0].y) - kn * (v[3].x - v[2].y);
+    // kspace_efield_idm's weight (nb_induction_model.f90:2560-2600), applied before the merge
+    const int kp = n - K.nlo, km = -n - K.nlo;
+    if (kp >= 0 && kp < K.len) {
+      const int k = K.kbeg + kp;
+      const double g = -4.0 * A.kv[k].ak;
+      atomicAdd(&A.sk[(size_t)k * 4 + 2 * A.par], g * pr);
+      atomicAdd(&A.sk[(size_t)k * 4 + 2 * A.par + 1], g * pi);
+    }
+    if (n > 0 && km >= 0 && km < K.len) {
+      const int k = K.kbeg + km;
+      const double g = -4.0 * A.kv[k].ak;
+      atomicAdd(&A.sk[(size_t)k * 4 + 2 * A.par], g * mr);
+      atomicAdd(&A.sk[(size_t)k * 4 + 2 * A.par + 1], g * mi);
     }
   }
 }
 
-// Gather and update of the row form: a block takes kRowSites sites and its warps take the
-// groups of rows in turn (kRowR rows per thread, 32 / kRowSites threads per site, so a warp
-// covers 32 / kRowSites x kRowR consecutive rows of the length-sorted list, whose n ranges are
-// close).  The block's Z factors are staged in shared memory before the wait for the step's
-// first kernel (they are fixed during the solve), and each warp stages the F(k) of a group's
-// rows before running over its n range, so that the loop reads only shared memory.  The
-// update is k_iter_b's.
-template <bool PCG>
-__global__ void __launch_bounds__(kRowWarps * 32, 768 / (kRowWarps * 32)) k_iter_b_rows(IterArgs A) {
-  constexpr int kSB = kRowSites, kRL = 32 / kRowSites, kG = kRL * kRowR;
-  // Z [n][site] of the block's sites (nz rows), then per warp the F(k) [row][n - nlo] of its
-  // group's kG rows (row stride row_span)
-  extern __shared__ double2 zsh[];
+// Gather and update: a block takes MT tiles of 8 sites, its warps the tiles of four rows in turn.
+// Per tile a lane builds the operands of its row and n (columns Re, Im of Q and of Q_z) from
+// S(n) and S(-n), loaded a tile ahead; then lane l holds Q and Q_z of site l / 4 and row l % 4
+// and contracts them with XY.  The sites' (cos, sin)(n z) stay in registers, loaded before the
+// wait for the step's first kernel.  The update is k_iter_b's.
+template <bool PCG, int J, int MT>
+__global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
+  constexpr int KS = 2 * J;  // steps of two n
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int si = lane % kSB, h = lane / kSB;
-  const int w0 = blockIdx.x * kSB;
-  const int ns_blk = min(kSB, A.nw - w0);
-  for (int u = threadIdx.x; u < A.nz * kSB; u += kRowWarps * 32) {
-    const int ni = u / kSB, s = u - ni * kSB;
-    zsh[u] = s < ns_blk ? A.ZT[(size_t)ni * A.nw + w0 + s] : make_double2(0.0, 0.0);
+  const int w0 = blockIdx.x * (8 * MT), ns_blk = min(8 * MT, A.nw - w0);
+  double zf[MT][KS];
+  int ws[MT];
+#pragma unroll
+  for (int m = 0; m < MT; m++) {
+    ws[m] = min(w0 + 8 * m + (lane >> 2), A.nw - 1);
+    const double *z = A.Zc + (size_t)ws[m] * A.zs + (lane & 3);
+#pragma unroll
+    for (int k = 0; k < KS; k++) zf[m][k] = z[4 * k];
   }
-  double *rns = reinterpret_cast<double *>(zsh + (size_t)A.nz * kSB);  // k_n by n + nmax
-  for (int u = threadIdx.x; u < A.nz; u += kRowWarps * 32) rns[u] = A.rn[u];
-  double2 *fsh = zsh + (size_t)A.nz * kSB + (A.nz + 1) / 2 + (size_t)wid * kG * A.row_span;
+  const int nt4 = (A.nrow + 3) / 4;
+  // operand element: row lane / 8 of the tile, column part ri (Re, Im), factor part cs (cos, sin)
+  const int ri = (lane >> 2) & 1, cs = lane & 1, n0 = (lane >> 1) & 1;
   pdl_wait();  // T.mu, S(k) and the step scalars of this step's first kernel
-  __syncthreads();  // the staged Z
   if (A.state[kIterFinished] != 0.0) return;  // finished in an earlier step of this pass
-  const int wc = w0 + (si < ns_blk ? si : 0);  // the site whose XY this lane reads
-  const double2 *skp = reinterpret_cast<const double2 *>(A.sk) + A.par;
-  const double2 *xyr = A.XYr + wc;
-  const double2 *zl = zsh + si + A.nmax * kSB;  // Z of n at zl[n * kSB]
-  double ex = 0.0, ey = 0.0, ez = 0.0;
-  const int ng = (A.nrow + kG - 1) / kG;
-  for (int g = wid; g < ng; g += kRowWarps) {
-    // the warp's rows g kG .. g kG + kG - 1: stage their F(k), then this lane's kRowR of them
-    const int gb = g * kG, gn = min(kG, A.nrow - gb);
-    __syncwarp();  // the previous group's reads of the staging buffer are done
-    for (int u = lane; u < gn * A.row_span; u += 32) {
-      const int r = u / A.row_span, j = u - r * A.row_span;
-      const KRow &K = A.rows[gb + r];
-      if (j < K.len) fsh[u] = skp[2 * (size_t)(K.kbeg + j)];
+  const double *sk = A.sk + 2 * A.par + (ri ^ cs);  // the part of S that the element combines
+  double ex[MT], ey[MT], ez[MT];
+#pragma unroll
+  for (int m = 0; m < MT; m++) ex[m] = ey[m] = ez[m] = 0.0;
+  double p[KS], q[KS];  // S(n) and S(-n)
+  int ks = 0, ks_next = 0;
+  auto load = [&](int t) {
+    const int r = 4 * t + (lane >> 3);
+    KRow K = A.rows[min(r, A.nrow - 1)];
+    ks_next = warp_max(K.nlo + K.len - 1) / 2 + 1;
+    if (r >= A.nrow) K.len = 0;
+#pragma unroll
+    for (int k = 0; k < KS; k++) {
+      const int n = 2 * k + n0, kp = n - K.nlo, km = -n - K.nlo;
+      p[k] = kp >= 0 && kp < K.len ? sk[(size_t)(K.kbeg + kp) * 4] : 0.0;
+      q[k] = n > 0 && km >= 0 && km < K.len ? sk[(size_t)(K.kbeg + km) * 4] : 0.0;
     }
-    __syncwarp();
-    const int rb = gb + h * kRowR;  // this lane's rows rb .. rb + kRowR - 1
-    int nlo[kRowR], len[kRowR];
-    int nb = INT_MAX, ne = INT_MIN;
+  };
+  if (wid < nt4) load(wid);
+  for (int t = wid; t < nt4; t += kRowWarps) {
+    ks = ks_next;
+    double bq[KS], bz[KS];
+    const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
 #pragma unroll
-    for (int r = 0; r < kRowR; r++) {
-      nlo[r] = len[r] = 0;
-      if (rb + r < A.nrow) {
-        const KRow &K = A.rows[rb + r];
-        nlo[r] = K.nlo;
-        len[r] = K.len;
-        nb = min(nb, nlo[r]);
-        ne = max(ne, nlo[r] + len[r]);
-      }
+    for (int k = 0; k < KS; k++) {
+      const double a = p[k] + q[k], d = p[k] - q[k];
+      bq[k] = sg * (cs == 0 ? a : d);
+      bz[k] = sg * (cs == 0 ? d : a) * A.rn[min(2 * k + n0, A.nmax) + A.nmax];
     }
-    // the warp runs the n range of all its rows
+    const int r2 = 4 * t + (lane & 3);
+    const KRow K2 = A.rows[min(r2, A.nrow - 1)];
+    double2 xy[MT];
 #pragma unroll
-    for (int o = kSB; o < 32; o <<= 1) {
-      nb = min(nb, __shfl_xor_sync(0xffffffffu, nb, o));
-      ne = max(ne, __shfl_xor_sync(0xffffffffu, ne, o));
-    }
-    const double2 *fl = fsh + (size_t)h * kRowR * A.row_span;
-    // this lane's XY factors of its rows, loaded now so that their latency overlaps the sums
-    double2 xy[kRowR];
+    for (int m = 0; m < MT; m++)
+      xy[m] = A.XYr[((size_t)(t >> 1) * A.nw + ws[m]) * 8 + 4 * (t & 1) + (lane & 3)];
+    if (t + kRowWarps < nt4) load(t + kRowWarps);
+    double2 Q[MT], Z[MT];
 #pragma unroll
-    for (int r = 0; r < kRowR; r++)
-      xy[r] = len[r] > 0 ? xyr[(size_t)(rb + r) * A.nw] : make_double2(0.0, 0.0);
-    double qx[kRowR], qy[kRowR], zx[kRowR], zy[kRowR];
+    for (int m = 0; m < MT; m++) Q[m] = Z[m] = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int r = 0; r < kRowR; r++) qx[r] = qy[r] = zx[r] = zy[r] = 0.0;
-#pragma unroll 2
-    for (int n = nb; n < ne; n++) {
-      const double2 z = zl[n * kSB];
-      const double rn = rns[n + A.nmax];
+    for (int k = 0; k < KS; k++)
+      if (k < ks)
 #pragma unroll
-      for (int r = 0; r < kRowR; r++) {
-        if ((unsigned)(n - nlo[r]) < (unsigned)len[r]) {
-          // kspace_efield_idm gather (nb_induction_model.f90:2560-2600): the phase times the
-          // conjugate of the weighted S(k), summed over the row
-          const double2 f = fl[r * A.row_span + (n - nlo[r])];
-          const double px = z.x * f.x + z.y * f.y, py = z.y * f.x - z.x * f.y;
-          qx[r] += px;
-          qy[r] += py;
-          zx[r] += rn * px;
-          zy[r] += rn * py;
+        for (int m = 0; m < MT; m++) {
+          dmma(Q[m], zf[m][k], bq[k]);
+          dmma(Z[m], zf[m][k], bz[k]);
         }
-      }
-    }
 #pragma unroll
-    for (int r = 0; r < kRowR; r++) {
-      if (len[r] > 0) {
-        const KRow &K = A.rows[rb + r];
-        const double a = xy[r].x * qx[r] - xy[r].y * qy[r];
-        ex += K.rl * a;
-        ey += K.rm * a;
-        ez += xy[r].x * zx[r] - xy[r].y * zy[r];
-      }
+    for (int m = 0; m < MT; m++) {  // rows past the last have XY = 0
+      const double a = xy[m].x * Q[m].x - xy[m].y * Q[m].y;
+      ex[m] += K2.rl * a;
+      ey[m] += K2.rm * a;
+      ez[m] += xy[m].x * Z[m].x - xy[m].y * Z[m].y;
     }
   }
   pdl_launch_dependents();  // the gather, the bulk of the kernel, is done
+  __shared__ double part[kRowWarps][3][8 * MT];
 #pragma unroll
-  for (int o = kSB; o < 32; o <<= 1) {
-    ex += __shfl_xor_sync(0xffffffffu, ex, o);
-    ey += __shfl_xor_sync(0xffffffffu, ey, o);
-    ez += __shfl_xor_sync(0xffffffffu, ez, o);
-  }
-  __shared__ double part[kRowWarps][3][kSB];
-  if (h == 0) {
-    part[wid][0][si] = ex;
-    part[wid][1][si] = ey;
-    part[wid][2][si] = ez;
+  for (int m = 0; m < MT; m++) {
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      ex[m] += __shfl_xor_sync(0xffffffffu, ex[m], o);
+      ey[m] += __shfl_xor_sync(0xffffffffu, ey[m], o);
+      ez[m] += __shfl_xor_sync(0xffffffffu, ez[m], o);
+    }
+    if ((lane & 3) == 0) {
+      part[wid][0][8 * m + (lane >> 2)] = ex[m];
+      part[wid][1][8 * m + (lane >> 2)] = ey[m];
+      part[wid][2][8 * m + (lane >> 2)] = ez[m];
+    }
   }
   __syncthreads();
   const auto ek = [&](int g, int c) {
@@ -955,26 +922,29 @@ cudaError_t launch_step(Kernel kernel, int blocks, const IterArgs &A, cudaStream
   return cudaLaunchKernelEx(&cfg, kernel, A);
 }
 
-// Dynamic shared memory of the row form's two kernels; the row form runs only where both fit
-// the default 48 KB per block (less the static arrays).
-size_t iter_rows_smem_a(int sum_sites, int row_span) {
-  return sizeof(double4) * (size_t)sum_sites +
-         sizeof(double2) * (size_t)sum_sites * (kRowTile + 1 + row_span);
-}
-size_t iter_rows_smem_b(int nz, int row_span) {
-  return sizeof(double2) * ((size_t)nz * kRowSites + (nz + 1) / 2 +
-                            (size_t)kRowWarps * 32 / kRowSites * kRowR * row_span);
-}
-bool iter_rows_fit(int sum_sites, int nz, int row_span) {
-  constexpr size_t kDefault = 48 * 1024 - 2048;  // room for the static shared arrays
-  return iter_rows_smem_a(sum_sites, row_span) <= kDefault &&
-         iter_rows_smem_b(nz, row_span) <= kDefault;
+// n tiles of four of the row form; it runs up to kRowTilesMax of them (k_max 19)
+int iter_row_tiles(int nmax) { return nmax / 4 + 1; }
+bool iter_rows_fit(int nmax) { return iter_row_tiles(nmax) <= kRowTilesMax; }
+
+// Sites of a structure-factor block: 96 (six steps per warp, their XY loaded ahead) while that
+// makes no more than a few waves of blocks, so that the atomics stay few; 48 in small boxes,
+// where blocks are too few otherwise.
+int iter_row_sites(int nw, int nrow) {
+  const int nt8 = (nrow + 7) / 8;
+  int cs = nw <= 512 ? 48 : 96;
+  while ((long long)nt8 * ((nw + cs - 1) / cs) > 148 * 8) cs *= 2;
+  return cs;
 }
 
 template <int J>
-cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, size_t smem, cudaStream_t st) {
-  return A.cu ? launch_step(k_iter_a_rows<true, J>, nb, A, st, smem)
-              : launch_step(k_iter_a_rows<false, J>, nb, A, st, smem);
+cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
+  const size_t smem = sizeof(double4) * A.row_sites + sizeof(double2) * kWarps * 4 * J * 32;
+  const auto k = A.cu ? k_iter_a_rows<true, J> : k_iter_a_rows<false, J>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_step(k, nb, A, st, smem);
 }
 
 cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st) {
@@ -982,15 +952,15 @@ cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st) {
   const int nA = (A.nw + kWarps - 1) / kWarps;
   const int nsc = (A.nw + A.sum_sites - 1) / A.sum_sites;
   if (A.rows) {
-    if (!iter_rows_fit(A.sum_sites, A.nz, A.row_span)) return cudaErrorInvalidValue;
-    const int ntile = (A.nrow + kRowTile - 1) / kRowTile;
-    const size_t smem = iter_rows_smem_a(A.sum_sites, A.row_span);
-    const int nb = nA + ntile * nsc;
-    const int j = (A.row_span + kRowLanes - 1) / kRowLanes;
-    if (j <= 2) return launch_iter_a_rows<2>(A, nb, smem, st);
-    if (j <= 4) return launch_iter_a_rows<4>(A, nb, smem, st);
-    if (j <= 8) return launch_iter_a_rows<8>(A, nb, smem, st);
-    return cudaErrorInvalidValue;
+    const int nb = nA + (A.nrow + 7) / 8 * ((A.nw + A.row_sites - 1) / A.row_sites);
+    switch (iter_row_tiles(A.nmax)) {
+      case 1: return launch_iter_a_rows<1>(A, nb, st);
+      case 2: return launch_iter_a_rows<2>(A, nb, st);
+      case 3: return launch_iter_a_rows<3>(A, nb, st);
+      case 4: return launch_iter_a_rows<4>(A, nb, st);
+      case 5: return launch_iter_a_rows<5>(A, nb, st);
+      default: return cudaErrorInvalidValue;
+    }
   }
   const size_t smem = sizeof(double) * 3 * A.sum_sites;
   const int nkt = (A.nk + kThreads - 1) / kThreads;
@@ -1013,13 +983,26 @@ cudaError_t launch_iter_b_gs(const IterArgs &A, cudaStream_t st) {
               : launch_step(k_iter_b<false, false, GS>, nb, A, st, 0, T);
 }
 
+template <int J>
+cudaError_t launch_iter_b_rows(const IterArgs &A, cudaStream_t st) {
+  // 16 sites per block once 8 make more than three waves of blocks: an operand then serves both
+  if (A.nw > 8 * 148 * 3)
+    return launch_step(A.cu ? k_iter_b_rows<true, J, 2> : k_iter_b_rows<false, J, 2>,
+                       (A.nw + 15) / 16, A, st, 0, kRowWarps * 32);
+  return launch_step(A.cu ? k_iter_b_rows<true, J, 1> : k_iter_b_rows<false, J, 1>, (A.nw + 7) / 8,
+                     A, st, 0, kRowWarps * 32);
+}
+
 cudaError_t launch_iter_b(const IterArgs &A, cudaStream_t st) {
   if (A.rows) {
-    if (!iter_rows_fit(A.sum_sites, A.nz, A.row_span)) return cudaErrorInvalidValue;
-    const int nb = (A.nw + kRowSites - 1) / kRowSites;
-    const size_t smem = iter_rows_smem_b(A.nz, A.row_span);
-    return A.cu ? launch_step(k_iter_b_rows<true>, nb, A, st, smem, kRowWarps * 32)
-                : launch_step(k_iter_b_rows<false>, nb, A, st, smem, kRowWarps * 32);
+    switch (iter_row_tiles(A.nmax)) {
+      case 1: return launch_iter_b_rows<1>(A, st);
+      case 2: return launch_iter_b_rows<2>(A, st);
+      case 3: return launch_iter_b_rows<3>(A, st);
+      case 4: return launch_iter_b_rows<4>(A, st);
+      case 5: return launch_iter_b_rows<5>(A, st);
+      default: return cudaErrorInvalidValue;
+    }
   }
   switch (A.gather_sites) {
     case 2: return launch_iter_b_gs<2>(A, st);
@@ -1032,16 +1015,17 @@ cudaError_t launch_iter_b(const IterArgs &A, cudaStream_t st) {
 }
 
 cudaError_t launch_phase_rows(const double2 *tab, int nm, SiteSets S, int kl, int km, int kn,
-                              const KRow *rows, int nrow, double2 *XYr, double2 *Z,
-                              double2 *ZT, cudaStream_t st) {
+                              const KRow *rows, int nrow, int zs, double2 *XYt, double *Zc,
+                              cudaStream_t st) {
   int k1 = kl > km ? kl : km;
   k1 = (k1 > kn ? k1 : kn) + 1;
   if (k1 < 2) k1 = 2;
-  const size_t total = (size_t)nm * S.np * ((size_t)nrow + 2 * kn + 1);
+  const size_t total = (size_t)nm * S.np * ((size_t)(nrow + 7) / 8 * 8 + zs / 2);
   if (total == 0) return cudaSuccess;
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  k_phase_rows<<<(unsigned)blocks, 256, 0, st>>>(tab, nm, S, k1, km, kn, rows, nrow, XYr, Z, ZT);
+  k_phase_rows<<<(unsigned)blocks, 256, 0, st>>>(tab, nm, S, k1, km, kn, rows, nrow, zs, XYt,
+                                                 reinterpret_cast<double2 *>(Zc));
   return cudaGetLastError();
 }
 
