@@ -26,6 +26,8 @@
 // reciprocal sums as matrix products over the rows of the k-vector list.  k_iter_a and k_iter_b
 // take them k-vector by k-vector, from the factor tables (k_max above the row form's) or, by
 // option, from the full phase matrix [site][k].
+#include <algorithm>
+
 #include "ccp_device.cuh"
 
 using namespace ccpd;
@@ -279,30 +281,95 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Blocks [0, nA) of a step's first kernel: T.mu, one warp per polarisable site; they also
+// Blocks [0, nA) of a step's first kernel: T.mu, two warps per polarisable site; they also
 // clear the S(k) buffer of the other step parity, whose last reader, the previous step's
-// gather, has finished.
+// gather, has finished.  The tensor entries are fixed during the solve, so a lane's first
+// kTmuPre entries (all of them at 9 A: 306 per site) and their source sites are loaded before
+// the wait for the previous step's dipoles; after it only the dipoles are.
+constexpr int kTmuWarps = 2, kTmuPre = 5;
+constexpr int kTmuSites = kWarps / kTmuWarps;  // sites per block
+__host__ __device__ constexpr int tmu_blocks(int nw) { return (nw + kTmuSites - 1) / kTmuSites; }
 template <bool PCG>
-__device__ __forceinline__ void iter_a_tmu(const IterArgs &A, const PcgIn &pin, int nA) {
+__device__ __forceinline__ void iter_a_tmu(const IterArgs &A, int block, int nA) {
+  const int w = block * kTmuSites + threadIdx.x / (32 * kTmuWarps);
+  const int lane = threadIdx.x % (32 * kTmuWarps);
+  const bool on = w < A.nw;
+  const int i = on ? w / A.np : 0, n_ent = on ? A.ncnt[i] * A.np : 0;
+  const size_t base = (size_t)w * A.cap * A.np;
+  const int *nb = A.nbr + (size_t)i * A.cap;
+  double4 t[kTmuPre + 1];
+  double b[kTmuPre + 1];
+  int src[kTmuPre + 1], q[kTmuPre + 1];
+#pragma unroll
+  for (int u = 0; u < kTmuPre; u++) {
+    const int e = lane + 32 * kTmuWarps * u;
+    t[u] = make_double4(0.0, 0.0, 0.0, 0.0);
+    b[u] = 0.0;
+    src[u] = q[u] = 0;
+    if (e < n_ent) {
+      const int n = e / A.np;
+      q[u] = e - n * A.np;
+      t[u] = A.T4[base + e];
+      b[u] = A.TB[base + e];
+      src[u] = nb[n] * A.np + q[u];
+    }
+  }
+  // the intramolecular entries
+  t[kTmuPre] = make_double4(0.0, 0.0, 0.0, 0.0);
+  b[kTmuPre] = 0.0;
+  src[kTmuPre] = q[kTmuPre] = 0;
+  if (on && lane < A.np) {
+    t[kTmuPre] = A.S4[(size_t)w * A.np + lane];
+    b[kTmuPre] = A.SB[(size_t)w * A.np + lane];
+    src[kTmuPre] = i * A.np + lane;
+    q[kTmuPre] = lane;
+  }
+  pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
+  PcgIn pin;
+  if constexpr (PCG) pin = pcg_in(A);
+  auto mu = [&](int s, int qs) {
+    if constexpr (PCG) return pin((size_t)s, qs);
+    else return MuIn{A.mu}((size_t)s, qs);
+  };
+  double ex = 0.0, ey = 0.0, ez = 0.0;
+  auto add = [&](const double4 &T, double B, const double3 &m) {
+    const double dm = T.w * (T.x * m.x + T.y * m.y + T.z * m.z);
+    ex += dm * T.x - B * m.x;
+    ey += dm * T.y - B * m.y;
+    ez += dm * T.z - B * m.z;
+  };
+  double3 m[kTmuPre + 1];
+#pragma unroll
+  for (int u = 0; u <= kTmuPre; u++) m[u] = mu(src[u], q[u]);  // site 0's where there is no entry
+#pragma unroll
+  for (int u = 0; u <= kTmuPre; u++) add(t[u], b[u], m[u]);
+#pragma unroll kTmuPre
+  for (int e = lane + 32 * kTmuWarps * kTmuPre; e < n_ent; e += 32 * kTmuWarps) {
+    const int n = e / A.np, qe = e - n * A.np;
+    add(A.T4[base + e], A.TB[base + e], mu(nb[n] * A.np + qe, qe));
+  }
   double2 *other = reinterpret_cast<double2 *>(A.sk) + (A.par ^ 1);
-  for (int k = blockIdx.x * kThreads + threadIdx.x; k < A.nk; k += nA * kThreads)
+  for (int k = block * kThreads + threadIdx.x; k < A.nk; k += nA * kThreads)
     other[2 * (size_t)k] = make_double2(0.0, 0.0);
-  const int w = blockIdx.x * kWarps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= A.nw) return;
-  double ex, ey, ez;
-  if constexpr (PCG)
-    tmu_warp(w, lane, A.nbr, A.ncnt, A.cap, A.np, A.T4, A.TB, A.S4, A.SB, pin, ex, ey, ez);
-  else
-    tmu_warp(w, lane, A.nbr, A.ncnt, A.cap, A.np, A.T4, A.TB, A.S4, A.SB, MuIn{A.mu}, ex, ey,
-             ez);
   // the next kernel may launch once every block is this far: late enough that its blocks
   // do not hold SM slots (which concurrent kernels could use) for long while they wait
   pdl_launch_dependents();
-  if (lane == 0) {
-    A.eim[(size_t)w * 3 + 0] = ex;
-    A.eim[(size_t)w * 3 + 1] = ey;
-    A.eim[(size_t)w * 3 + 2] = ez;
+  ex = warp_sum(ex);
+  ey = warp_sum(ey);
+  ez = warp_sum(ez);
+  __shared__ double part[kWarps][3];
+  const int wid = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    part[wid][0] = ex;
+    part[wid][1] = ey;
+    part[wid][2] = ez;
+  }
+  __syncthreads();
+  if (on && lane < 3) {
+    double v = 0.0;
+#pragma unroll
+    for (int u = 0; u < kTmuWarps; u++) v += part[wid + u][lane];
+    A.eim[(size_t)w * 3 + lane] = v;
   }
 }
 
@@ -311,14 +378,14 @@ __global__ void __launch_bounds__(kThreads)
     k_iter_a(IterArgs A) {
   // no test of the finished flag here: a step after the finish only rewrites the T.mu
   // scratch and S(k), which the next use clears, and it saves a dependent load per step
-  pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
-  const int nA = (A.nw + kWarps - 1) / kWarps;
-  PcgIn pin;
-  if constexpr (PCG) pin = pcg_in(A);
+  const int nA = tmu_blocks(A.nw);
   if ((int)blockIdx.x < nA) {
-    iter_a_tmu<PCG>(A, pin, nA);
+    iter_a_tmu<PCG>(A, blockIdx.x, nA);
     return;
   }
+  pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
+  PcgIn pin;
+  if constexpr (PCG) pin = pcg_in(A);
   // structure factors: block b covers k-vectors [kt*256, kt*256+256) and sites of chunk sc
   extern __shared__ double smu[];  // A.sum_sites x 3 dipole components
   const int b = blockIdx.x - nA;
@@ -575,7 +642,7 @@ __device__ __forceinline__ void dmma(double2 &d, double a, double b) {
 }
 
 constexpr int kRowSteps = 6;  // steps of four sites whose XY a warp loads before it waits
-constexpr int kRowWarps = 8;  // warps of a gather block, each taking row tiles in turn
+constexpr int kRowWarps = 8;  // warps of a gather block, taking row tiles in turn
 
 // the largest n of the rows of a lane's tile (rows sorted by length: only the row (0, 0), which
 // has no n < 1, can reach further than its neighbours)
@@ -587,19 +654,22 @@ __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffff
 // warps' partial sums meet in shared memory, and one thread per (row, n) combines them into
 // S(r, n) and S(r, -n), merged with FP64 atomics as in k_iter_a.  The first steps' XY are
 // loaded before the wait for the previous step (the tables are fixed during the solve).
-template <bool PCG, int J>
+template <bool PCG, int J, bool ZS>
 __global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
-  const int nA = (A.nw + kWarps - 1) / kWarps;
-  if ((int)blockIdx.x < nA) {
-    pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
-    PcgIn pin;
-    if constexpr (PCG) pin = pcg_in(A);
-    iter_a_tmu<PCG>(A, pin, nA);
+  // the sums' blocks first: they run longest.  The loop took 594 / 3682 us with T.mu's blocks
+  // first, 565 / 3560 with the two alternating and 561 / 3400 so (512 / 2048 waters).
+  const int nA = tmu_blocks(A.nw), nR = gridDim.x - nA;
+  if ((int)blockIdx.x >= nR) {
+    iter_a_tmu<PCG>(A, blockIdx.x - nR, nA);
     return;
   }
-  extern __shared__ double4 smu4[];  // A.row_sites dipoles, then the warps' sums
-  double2(*red)[4 * J][32] = reinterpret_cast<double2(*)[4 * J][32]>(smu4 + A.row_sites);
-  const int b = blockIdx.x - nA, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // A.row_sites dipoles; the sites' Zc (rows of 8 J + 2: no bank conflicts between the four
+  // sites of a step), and in the same place at the end the warps' sums
+  extern __shared__ double4 smu4[];
+  constexpr int kZs = 8 * J + 2;
+  double *zsm = reinterpret_cast<double *>(smu4 + A.row_sites);
+  double2(*red)[4 * J][32] = reinterpret_cast<double2(*)[4 * J][32]>(zsm);
+  const int b = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nt8 = (A.nrow + 7) / 8, rt = b % nt8, s0 = b / nt8 * A.row_sites;
   const int r = min(rt * 8 + (lane >> 2), A.nrow - 1);
   const KRow R = A.rows[r];
@@ -611,6 +681,12 @@ __global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
 #pragma unroll
   for (int t = 0; t < kRowSteps; t++)
     xy[t] = xyt[(size_t)min(s0 + q0 + 4 * t, A.nw - 1) * 8];
+  if constexpr (ZS)
+    for (int u = threadIdx.x; u < A.row_sites * 4 * J; u += kThreads) {
+      const int q = u / (4 * J), c = u - q * (4 * J);
+      reinterpret_cast<double2 *>(zsm + q * kZs)[c] =
+          reinterpret_cast<const double2 *>(A.Zc + (size_t)min(s0 + q, A.nw - 1) * A.zs)[c];
+    }
   pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
   PcgIn pin;
   if constexpr (PCG) pin = pcg_in(A);
@@ -637,8 +713,9 @@ __global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
 #pragma unroll
     for (int t = 0; t < kRowSteps; t++) {
       if (t0 + t < steps) {  // warp-uniform
-        const int q = q0 + 4 * (t0 + t), w = min(s0 + q, A.nw - 1);  // mu = 0 past the last site
-        const double *z = A.Zc + (size_t)w * A.zs + (lane >> 2);
+        const int q = q0 + 4 * (t0 + t);  // mu = 0 past the last site
+        const double *z = (ZS ? zsm + q * kZs
+                              : A.Zc + (size_t)min(s0 + q, A.nw - 1) * A.zs) + (lane >> 2);
         double zf[J];
 #pragma unroll
         for (int j = 0; j < J; j++) zf[j] = j < jt ? z[8 * j] : 0.0;
@@ -658,6 +735,7 @@ __global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
         xy[t] = xyt[(size_t)min(s0 + q0 + 4 * (t0 + kRowSteps + t), A.nw - 1) * 8];
   }
   pdl_launch_dependents();
+  if constexpr (ZS) __syncthreads();  // every warp has read its sites' Zc
 #pragma unroll
   for (int c = 0; c < 4; c++)
 #pragma unroll
@@ -705,8 +783,9 @@ __global__ void __launch_bounds__(kThreads) k_iter_a_rows(IterArgs A) {
 // Gather and update: a block takes MT tiles of 8 sites, its warps the tiles of four rows in turn.
 // Per tile a lane builds the operands of its row and n (columns Re, Im of Q and of Q_z) from
 // S(n) and S(-n), loaded a tile ahead; then lane l holds Q and Q_z of site l / 4 and row l % 4
-// and contracts them with XY.  The sites' (cos, sin)(n z) stay in registers, loaded before the
-// wait for the step's first kernel.  The update is k_iter_b's.
+// and contracts them with XY.  The sites' (cos, sin)(n z) stay in registers; they and the first
+// tile's XY and row are loaded before the wait for the step's first kernel, and the values of
+// the update right after it.  The update is k_iter_b's.
 template <bool PCG, int J, int MT>
 __global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
   constexpr int KS = 2 * J;  // steps of two n
@@ -724,19 +803,31 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
   const int nt4 = (A.nrow + 3) / 4;
   // operand element: row lane / 8 of the tile, column part ri (Re, Im), factor part cs (cos, sin)
   const int ri = (lane >> 2) & 1, cs = lane & 1, n0 = (lane >> 1) & 1;
-  pdl_wait();  // T.mu, S(k) and the step scalars of this step's first kernel
-  if (A.state[kIterFinished] != 0.0) return;  // finished in an earlier step of this pass
   const double *sk = A.sk + 2 * A.par + (ri ^ cs);  // the part of S that the element combines
-  double ex[MT], ey[MT], ez[MT];
+  double kn[KS];  // k_n, with the sign of the element's Q_z
+  const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
 #pragma unroll
-  for (int m = 0; m < MT; m++) ex[m] = ey[m] = ez[m] = 0.0;
-  double p[KS], q[KS];  // S(n) and S(-n)
-  int ks = 0, ks_next = 0;
-  auto load = [&](int t) {
+  for (int k = 0; k < KS; k++) kn[k] = sg * A.rn[min(2 * k + n0, A.nmax) + A.nmax];
+  double2 xy[MT];
+  double rl = 0.0, rm = 0.0;
+  KRow K{};
+  int ks_next = 0;
+  auto load_rows = [&](int t) {  // fixed during the solve
+    const KRow &R = A.rows[min(4 * t + (lane & 3), A.nrow - 1)];
+    rl = R.rl;
+    rm = R.rm;
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+      xy[m] = A.XYr[((size_t)(t >> 1) * A.nw + ws[m]) * 8 + 4 * (t & 1) + (lane & 3)];
+  };
+  auto load_row = [&](int t) {
     const int r = 4 * t + (lane >> 3);
-    KRow K = A.rows[min(r, A.nrow - 1)];
+    K = A.rows[min(r, A.nrow - 1)];
     ks_next = warp_max(K.nlo + K.len - 1) / 2 + 1;
     if (r >= A.nrow) K.len = 0;
+  };
+  double p[KS], q[KS];  // S(n) and S(-n)
+  auto load_s = [&]() {
 #pragma unroll
     for (int k = 0; k < KS; k++) {
       const int n = 2 * k + n0, kp = n - K.nlo, km = -n - K.nlo;
@@ -744,24 +835,35 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
       q[k] = n > 0 && km >= 0 && km < K.len ? sk[(size_t)(K.kbeg + km) * 4] : 0.0;
     }
   };
-  if (wid < nt4) load(wid);
+  if (wid < nt4) {
+    load_row(wid);
+    load_rows(wid);
+  }
+  pdl_wait();  // T.mu, S(k) and the step scalars of this step's first kernel
+  const double finished = A.state[kIterFinished];
+  if (wid < nt4) load_s();
+  if (finished != 0.0) return;  // finished in an earlier step of this pass
+  double ex[MT], ey[MT], ez[MT];
+#pragma unroll
+  for (int m = 0; m < MT; m++) ex[m] = ey[m] = ez[m] = 0.0;
   for (int t = wid; t < nt4; t += kRowWarps) {
-    ks = ks_next;
+    const int ks = ks_next;
     double bq[KS], bz[KS];
-    const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
 #pragma unroll
     for (int k = 0; k < KS; k++) {
       const double a = p[k] + q[k], d = p[k] - q[k];
       bq[k] = sg * (cs == 0 ? a : d);
-      bz[k] = sg * (cs == 0 ? d : a) * A.rn[min(2 * k + n0, A.nmax) + A.nmax];
+      bz[k] = kn[k] * (cs == 0 ? d : a);
     }
-    const int r2 = 4 * t + (lane & 3);
-    const KRow K2 = A.rows[min(r2, A.nrow - 1)];
-    double2 xy[MT];
+    double2 x[MT];
 #pragma unroll
-    for (int m = 0; m < MT; m++)
-      xy[m] = A.XYr[((size_t)(t >> 1) * A.nw + ws[m]) * 8 + 4 * (t & 1) + (lane & 3)];
-    if (t + kRowWarps < nt4) load(t + kRowWarps);
+    for (int m = 0; m < MT; m++) x[m] = xy[m];
+    const double l = rl, mm = rm;
+    if (t + kRowWarps < nt4) {
+      load_row(t + kRowWarps);
+      load_s();
+      load_rows(t + kRowWarps);
+    }
     double2 Q[MT], Z[MT];
 #pragma unroll
     for (int m = 0; m < MT; m++) Q[m] = Z[m] = make_double2(0.0, 0.0);
@@ -775,10 +877,10 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
         }
 #pragma unroll
     for (int m = 0; m < MT; m++) {  // rows past the last have XY = 0
-      const double a = xy[m].x * Q[m].x - xy[m].y * Q[m].y;
-      ex[m] += K2.rl * a;
-      ey[m] += K2.rm * a;
-      ez[m] += xy[m].x * Z[m].x - xy[m].y * Z[m].y;
+      const double a = x[m].x * Q[m].x - x[m].y * Q[m].y;
+      ex[m] += l * a;
+      ey[m] += mm * a;
+      ez[m] += x[m].x * Z[m].x - x[m].y * Z[m].y;
     }
   }
   pdl_launch_dependents();  // the gather, the bulk of the kernel, is done
@@ -936,10 +1038,17 @@ int iter_row_sites(int nw, int nrow) {
   return cs;
 }
 
+// Up to this many sites per block, their Zc fit the shared memory that the warps' sums take
+// at the end; longer blocks read them from memory, where they overlap with the products.
+constexpr int kRowStage = 96;
 template <int J>
 cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
-  const size_t smem = sizeof(double4) * A.row_sites + sizeof(double2) * kWarps * 4 * J * 32;
-  const auto k = A.cu ? k_iter_a_rows<true, J> : k_iter_a_rows<false, J>;
+  const bool zs = A.row_sites <= kRowStage;
+  const size_t smem = sizeof(double4) * A.row_sites +
+                      std::max(sizeof(double2) * kWarps * 4 * J * 32,
+                               zs ? sizeof(double) * (size_t)A.row_sites * (8 * J + 2) : 0);
+  const auto k = zs ? (A.cu ? k_iter_a_rows<true, J, true> : k_iter_a_rows<false, J, true>)
+                    : (A.cu ? k_iter_a_rows<true, J, false> : k_iter_a_rows<false, J, false>);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -949,7 +1058,7 @@ cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
 
 cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st) {
   if (A.sum_sites < 1 || A.sum_sites > kSumSitesMax) return cudaErrorInvalidValue;
-  const int nA = (A.nw + kWarps - 1) / kWarps;
+  const int nA = tmu_blocks(A.nw);
   const int nsc = (A.nw + A.sum_sites - 1) / A.sum_sites;
   if (A.rows) {
     const int nb = nA + (A.nrow + 7) / 8 * ((A.nw + A.row_sites - 1) / A.row_sites);
