@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -170,6 +171,8 @@ struct ccp_context {
   double *d_istate = nullptr;  // kIterStateLen slots (IterStateSlot)
   double *h_istate = nullptr;
   unsigned *d_ticket = nullptr;  // last-block ticket of the fused update kernel
+  std::array<int, 5> clu_key{};  // sizes that clu_fits was asked for
+  bool clu_fits = false;         // the solve in one cluster applies to them
   int ind_per_iter = 0;          // kernels per Jacobi iteration of the last solve
   std::vector<long long> ind_key;
   // phase factors of the polarisable sites for the dipole iteration (k_iter.cu), when they
@@ -666,6 +669,16 @@ int ensure_ind_graph(ccp_context *c) {
   return CCP_OK;
 }
 
+// Whether the solve takes the one-cluster form (k_iter.cu).
+bool dip_cluster(ccp_context *c, const IterArgs &A) {
+  const std::array<int, 5> key = {A.nw, A.nrow, A.nmax, A.rows != nullptr, A.cu != nullptr};
+  if (key != c->clu_key) {
+    c->clu_fits = dip_cluster_fits(A);
+    c->clu_key = key;
+  }
+  return c->clu_fits;
+}
+
 // The whole Jacobi solve from mu = 0.  The state {iterations, change, energy} is copied to
 // h_istate; in the graph form the copy completes at the evaluation's final synchronisation.
 int run_dipole_loop(ccp_context *c, cudaStream_t st) {
@@ -673,6 +686,13 @@ int run_dipole_loop(ccp_context *c, cudaStream_t st) {
   const bool pcg = pcg_solver(c);
   c->pcg_active = pcg;
   if (pcg && !c->d_pcg) CK(dalloc(&c->d_pcg, 4 * (size_t)c->nm * c->S.np * 3));
+  const IterArgs A1 = make_iter_args(c, 0, 0, 0);
+  if (c->opt_graph && dip_cluster(c, A1)) {
+    if (!cuda_ok(launch_dip_cluster(A1, st), "dipole solve")) return CCP_ERR_CUDA;
+    CK(cudaMemcpyAsync(c->h_istate, c->d_istate, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    c->ind_per_iter = 0;
+    return CCP_OK;
+  }
   const double thr = ind_threshold(c);
   CK(cudaMemsetAsync(c->d_istate, 0, kIterStateLen * sizeof(double), st));
   CK(cudaMemsetAsync(c->d_scal + S_IND_CHANGE, 0, 2 * sizeof(double), st));
@@ -1712,6 +1732,8 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
     *value = ctx->opt_rows;
   } else if (n == "dipole_row_form_active") {
     *value = ctx->use_rows ? 1 : 0;
+  } else if (n == "dipole_cluster_active") {
+    *value = ctx->opt_graph && ctx->clu_fits;
   } else if (n == "dipole_solver") {
     *value = ctx->opt_solver;
   } else if (n == "cell_list") {

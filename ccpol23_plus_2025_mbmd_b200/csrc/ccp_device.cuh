@@ -332,6 +332,11 @@ cudaError_t launch_phase_matrix(const KGather *kg, int nk, int nw, int nlm, int 
 cudaError_t launch_dip_first(const IterArgs &A, cudaStream_t st);
 // Start of the PCG form of the solve (A.cu.. set): x = 0, u = alpha E0, state cleared.
 cudaError_t launch_pcg_first(const IterArgs &A, cudaStream_t st);
+// The whole Jacobi solve (first step included) as one thread-block cluster, for small boxes:
+// whether the form takes these sizes on the current device (asked once per set of sizes: it
+// queries the device), and its launch.
+bool dip_cluster_fits(const IterArgs &A);
+cudaError_t launch_dip_cluster(const IterArgs &A, cudaStream_t st);
 cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st);
 cudaError_t launch_iter_b(const IterArgs &A, cudaStream_t st);
 cudaError_t launch_pair_indforce(const double *x, const double *y, const double *z,

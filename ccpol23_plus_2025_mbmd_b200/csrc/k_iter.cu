@@ -22,10 +22,13 @@
 //      of a graph body that unrolls several steps then returns at once) and, inside the
 //      graph, sets the WHILE node's condition.  S(k) alternates between two buffers by step
 //      parity, so no block has to clear it after the gather.
-// The step normally runs in the row form (k_iter_a_rows, k_iter_b_rows below), which takes the
+// Small boxes run the whole solve in one cluster instead (k_dip_cluster).  The step normally
+// runs in the row form (k_iter_a_rows, k_iter_b_rows below), which takes the
 // reciprocal sums as matrix products over the rows of the k-vector list.  k_iter_a and k_iter_b
 // take them k-vector by k-vector, from the factor tables (k_max above the row form's) or, by
 // option, from the full phase matrix [site][k].
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "ccp_device.cuh"
@@ -911,6 +914,351 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_iter_b_rows(IterArgs A) {
     jacobi_update(A, w0, ns_blk, ek);
 }
 
+// ------------------------------------------------------------------ the solve in one cluster
+// Small boxes: the whole Jacobi solve as one kernel, a thread-block cluster whose blocks own ns
+// polarisable sites each.  A step of so few sites is a chain of latencies (two launches, the
+// loads after them, atomics and a ticket: 10.5 us at 37 waters, of which the sums take less
+// than one).  Here every block holds what it needs of the tables for the whole solve in shared
+// memory (its sites' tensor entries and phase factors, one row tile's phase factors of all
+// sites), all dipoles and all S(k) combinations; it receives the other blocks' parts of those
+// by distributed shared memory, and a step has two cluster barriers:
+//   - four warps take the block's (row tile, n tile), a share of the sites each, as in
+//     k_iter_a_rows; the others take T.mu of the block's sites;
+//   - barrier; the gather of the block's sites, a tile of four rows per warp, as in
+//     k_iter_b_rows, and the update; barrier.
+// The change of a step is summed beside the next step's first half, which is thrown away after
+// the last one.  Every block forms the total from the blocks' sums in the same order, so all
+// leave together.
+// 37 waters, 27 steps: 139 us (275 as step kernels); what remains is latency, 5 us a step, of
+// which 1.8 are the two barriers with the stores that they wait for.  The form ends where a
+// block's tables no longer fit its shared memory (some 45 waters): with the tables left in
+// global memory a step took longer than its two kernels (473 us against 327 at 128 waters).
+constexpr int kCluThreads = 512, kCluWarps = kCluThreads / 32, kCluRowWarps = 4;
+constexpr int kCluTiles = 2;  // site tiles of 8 per block, at most
+constexpr int kCluMax = 16;   // blocks of the cluster
+static_assert(kCluMax * kCluTiles <= 32, "a lane per block and tile");
+constexpr size_t kCluSmem = 227 * 1024 - 64;
+
+__host__ __device__ constexpr int clu_sites(int nw) { return ((nw + kCluMax - 1) / kCluMax + 7) / 8 * 8; }
+constexpr int kCluRed = kCluWarps * 3 * 8 * kCluTiles > kCluRowWarps * 4 * 64
+                            ? kCluWarps * 3 * 8 * kCluTiles
+                            : kCluRowWarps * 4 * 64;
+struct CluSmem {  // offsets in doubles
+  int ld, nwp, mu, ad, red, xyt, zt, xy, z, t4, tb, src, eim, slot, total;
+  __host__ __device__ CluSmem(int J, int nw, int nrow) {
+    const int ns = clu_sites(nw), nr8 = (nrow + 7) / 8 * 8;
+    ld = 16 * J + 8;  // 64 bytes past a multiple of 128: two rows' elements in distinct banks
+    nwp = (nw + 31) / 32 * 32;  // sites and tensor entries, padded with zeros
+    mu = 0;                              // double4 [nwp]
+    t4 = mu + 4 * nwp;                   // double4 [ns][nwp]: a site's entries, at most one per site
+    ad = t4 + 4 * ns * nwp;              // [nr8][ld]: (S(n) + S(-n), S(n) - S(-n))
+    red = ad + nr8 * ld;                 // the warps' sums, of either half step
+    xyt = red + kCluRed;                 // double2 [nw][8]: the row tile's
+    zt = xyt + 16 * nw;                  // [nw][8]: the n tile's
+    xy = zt + 8 * nw;         // double2 [nr8][ns]: the block's sites'
+    z = xy + 2 * nr8 * ns;               // [ns][8 J + 2]
+    tb = z + ns * (8 * J + 2);           // [ns][nwp]
+    src = tb + ns * nwp;                 // int [ns][nwp]
+    eim = src + ns * nwp / 2;            // [ns][4]
+    slot = eim + 4 * ns;                 // [2][32] change by step parity, [32] energy, the flag
+    total = slot + 3 * 32 + 2;
+  }
+};
+
+template <int J>
+__global__ void __launch_bounds__(kCluThreads) k_dip_cluster(IterArgs A) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ double4 clu4[];
+  double *sm = reinterpret_cast<double *>(clu4);
+  const int me = (int)cl.block_rank();
+  const CluSmem L(J, A.nw, A.nrow);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = A.nw;
+  const int ns = clu_sites(nw), w0 = me * ns, nloc = min(max(nw - w0, 0), ns);
+  const int nt8 = (A.nrow + 7) / 8, nt4 = (A.nrow + 3) / 4, mt = ns / 8;
+  double4 *mu = clu4, *T4 = reinterpret_cast<double4 *>(sm + L.t4);
+  double *AD = sm + L.ad, *Zt = sm + L.zt, *Zs = sm + L.z, *TB = sm + L.tb, *eim = sm + L.eim;
+  double2(*red)[4][32] = reinterpret_cast<double2(*)[4][32]>(sm + L.red);
+  double(*part)[3][8 * kCluTiles] = reinterpret_cast<double(*)[3][8 * kCluTiles]>(sm + L.red);
+  double2 *XYt = reinterpret_cast<double2 *>(sm + L.xyt), *XYs = reinterpret_cast<double2 *>(sm + L.xy);
+  int *src = reinterpret_cast<int *>(sm + L.src);
+  double *slot = sm + L.slot;
+  volatile int *more = reinterpret_cast<int *>(slot + 3 * 32);
+  constexpr int kZs = 8 * J + 2, KS = 2 * J;
+  const int rt = me % nt8, jn = me / nt8;  // the block's row tile and n tile
+  const bool rows_here = jn < J;
+
+  // ---- the tables, and the first step from mu = 0 (as k_dip_first) in every block alike
+  double ch = 0.0, en = 0.0;
+  for (int w = tid; w < L.nwp; w += kCluThreads) {
+    double m[3] = {0.0, 0.0, 0.0};
+    if (w < nw) {
+      const double polr = A.S.apol[w % A.np];
+      double E0[3];
+      for (int c = 0; c < 3; c++) {
+        E0[c] = A.e0[(size_t)w * 3 + c];
+        m[c] = polr * E0[c];
+        ch += m[c] * m[c];
+      }
+      en += -0.5 * polr * (E0[0] * E0[0] + E0[1] * E0[1] + E0[2] * E0[2]);
+    }
+    mu[w] = make_double4(m[0], m[1], m[2], 0.0);
+  }
+  ch = warp_sum(ch);
+  en = warp_sum(en);
+  double *wsum = sm + L.red;
+  if (lane == 0) {
+    wsum[wid] = ch;
+    wsum[kCluWarps + wid] = en;
+  }
+  for (int g = wid; g < nloc; g += kCluWarps) {
+    const int w = w0 + g, i = w / A.np;
+    const int n_ent = min(A.ncnt[i] * A.np, nw - A.np);
+    const size_t base = (size_t)w * A.cap * A.np;
+    for (int e = lane; e < L.nwp; e += 32) {
+      double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
+      double b = 0.0;
+      int q = 0;
+      if (e < A.np) {  // the intramolecular entries first
+        t = A.S4[(size_t)w * A.np + e];
+        b = A.SB[(size_t)w * A.np + e];
+        q = i * A.np + e;
+      } else if (e - A.np < n_ent) {
+        const int n = (e - A.np) / A.np;
+        t = A.T4[base + e - A.np];
+        b = A.TB[base + e - A.np];
+        q = A.nbr[(size_t)i * A.cap + n] * A.np + (e - A.np) - n * A.np;
+      }
+      T4[g * L.nwp + e] = t;
+      TB[g * L.nwp + e] = b;
+      src[g * L.nwp + e] = q;
+    }
+  }
+  if (rows_here) {
+    for (int u = tid; u < nw * 8; u += kCluThreads) XYt[u] = A.XYr[(size_t)rt * nw * 8 + u];
+    for (int u = tid; u < nw * 8; u += kCluThreads) Zt[u] = A.Zc[(size_t)(u >> 3) * A.zs + 8 * jn + (u & 7)];
+  }
+  for (int u = tid; u < nt8 * 8 * ns; u += kCluThreads) {
+    const int r = u / ns, g = u - r * ns;
+    XYs[u] = A.XYr[((size_t)(r >> 3) * nw + min(w0 + g, nw - 1)) * 8 + (r & 7)];
+  }
+  for (int u = tid; u < ns * 8 * J; u += kCluThreads) {
+    const int g = u / (8 * J), c = u - g * (8 * J);
+    Zs[g * kZs + c] = A.Zc[(size_t)min(w0 + g, nw - 1) * A.zs + c];
+  }
+  for (int u = tid; u < nt8 * 8 * L.ld; u += kCluThreads) AD[u] = 0.0;
+  // structure factors: the lane's row, the warp's sites, and the thread's (row, n) at the end
+  double rl = 0.0, rm = 0.0, kn_a = 0.0, gp = 0.0, gm = 0.0;
+  const int fin_row = rt * 8 + (lane >> 2), fin_n = 4 * jn + (lane & 3);
+  bool fin = false;
+  if (rows_here && wid < kCluRowWarps) {
+    const KRow R = A.rows[min(fin_row, A.nrow - 1)];
+    rl = R.rl;
+    rm = R.rm;
+    fin = fin_row < A.nrow && fin_n <= A.nmax;
+    if (fin) {
+      const int kp = fin_n - R.nlo, km = -fin_n - R.nlo;
+      kn_a = A.rn[fin_n + A.nmax];
+      // kspace_efield_idm's weights (nb_induction_model.f90:2560-2600)
+      if (kp >= 0 && kp < R.len) gp = -4.0 * A.kv[R.kbeg + kp].ak;
+      if (fin_n > 0 && km >= 0 && km < R.len) gm = -4.0 * A.kv[R.kbeg + km].ak;
+    }
+  }
+  const int spw = ((nw + kCluRowWarps - 1) / kCluRowWarps + 3) / 4 * 4;  // sites of a row warp
+  const int q0 = wid * spw + (lane & 3);
+  const int steps = wid < kCluRowWarps ? min(spw, max(nw - wid * spw, 0) + 3) / 4 : 0;
+  // gather: the warp's tile of four rows
+  const int ri = (lane >> 2) & 1, cs = lane & 1, n0 = (lane >> 1) & 1;
+  const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
+  const double *ad = AD + (4 * wid + (lane >> 3)) * L.ld + 4 * n0 + (ri ^ cs);
+  double gl = 0.0, gmm = 0.0, kn[KS];
+  int ks = 0;
+  if (wid < nt4) {
+    const KRow K = A.rows[min(4 * wid + (lane >> 3), A.nrow - 1)];
+    ks = warp_max(K.nlo + K.len - 1) / 2 + 1;
+    const KRow R = A.rows[min(4 * wid + (lane & 3), A.nrow - 1)];
+    gl = R.rl;
+    gmm = R.rm;
+  }
+#pragma unroll
+  for (int k = 0; k < KS; k++) kn[k] = sg * A.rn[min(2 * k + n0, A.nmax) + A.nmax];
+  // update: warp m takes site tile m, lane (component, site)
+  const int uc = lane >> 3, ug = 8 * wid + (lane & 7), uw = w0 + ug;
+  const bool upd = wid < mt && uc < 3 && ug < nloc;
+  const double polr = upd ? A.S.apol[uw % A.np] : 0.0;
+  const double e0 = upd ? A.e0[(size_t)uw * 3 + uc] : 0.0;
+  __syncthreads();
+  double chg = 0.0, ene = 0.0;  // of step `it`
+  for (int u = 0; u < kCluWarps; u++) {
+    chg += wsum[u];
+    ene += wsum[kCluWarps + u];
+  }
+  int it = 1;
+  double e_up = 0.0;  // the lane's part of the energy of its last update
+  cl.sync();  // every block runs and has its combinations cleared
+  while (it > 1 || (chg > A.thr && it < A.maxit)) {
+    if (wid < kCluRowWarps) {
+      if (rows_here) {
+        double2 acc[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[c] = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int t = 0; t < steps; t++) {
+          const int q = q0 + 4 * t, w = min(q, nw - 1);  // mu = 0 past the last site
+          const double2 xy = XYt[w * 8 + (lane >> 2)];
+          const double zf = Zt[w * 8 + (lane >> 2)];
+          const double4 m = mu[q];
+          const double d = rl * m.x + rm * m.y;
+          dmma(acc[0], xy.x * d, zf);
+          dmma(acc[1], xy.y * d, zf);
+          dmma(acc[2], xy.x * m.z, zf);
+          dmma(acc[3], xy.y * m.z, zf);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) red[wid][c][lane] = acc[c];
+        asm volatile("bar.sync 1, %0;" ::"n"(kCluRowWarps * 32) : "memory");
+        if (fin) {  // in every row warp alike, which serves a share of the blocks
+          double2 v[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            double2 x[kCluRowWarps];
+#pragma unroll
+            for (int w = 0; w < kCluRowWarps; w++) x[w] = red[w][c][lane];
+            v[c].x = (x[0].x + x[1].x) + (x[2].x + x[3].x);
+            v[c].y = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+          }
+          // B + k_n C (n), B - k_n C (-n), times cos +- i sin
+          const double pr = gp * ((v[0].x - v[1].y) + kn_a * (v[2].x - v[3].y));
+          const double pi = gp * ((v[0].y + v[1].x) + kn_a * (v[2].y + v[3].x));
+          const double mr = gm * ((v[0].x + v[1].y) - kn_a * (v[2].x + v[3].y));
+          const double mi = gm * ((v[1].x - v[0].y) - kn_a * (v[3].x - v[2].y));
+          const double4 o = make_double4(pr + mr, pi + mi, pr - mr, pi - mi);
+          double4 *at = reinterpret_cast<double4 *>(AD + fin_row * L.ld + 4 * fin_n);
+#pragma unroll
+          for (int b = 0; b < kCluMax; b += kCluRowWarps) *cl.map_shared_rank(at, b + wid) = o;
+        }
+      }
+    } else {
+      for (int g = wid - kCluRowWarps; g < nloc; g += kCluWarps - kCluRowWarps) {
+        double ex = 0.0, ey = 0.0, ez = 0.0;
+#pragma unroll 4
+        for (int e = lane; e < L.nwp; e += 32) {
+          const double4 T = T4[g * L.nwp + e], m = mu[src[g * L.nwp + e]];
+          const double B = TB[g * L.nwp + e], dm = T.w * (T.x * m.x + T.y * m.y + T.z * m.z);
+          ex += dm * T.x - B * m.x;
+          ey += dm * T.y - B * m.y;
+          ez += dm * T.z - B * m.z;
+        }
+        ex = warp_sum(ex);
+        ey = warp_sum(ey);
+        ez = warp_sum(ez);
+        if (lane == 0) {
+          eim[4 * g] = ex;
+          eim[4 * g + 1] = ey;
+          eim[4 * g + 2] = ez;
+        }
+      }
+    }
+    cl.sync();  // all combinations are here, and no block reads the dipoles any more
+    {
+      double bq[KS], bz[KS];
+#pragma unroll
+      for (int k = 0; k < KS; k++) {
+        const double a = wid < nt4 ? ad[8 * k] : 0.0, d = wid < nt4 ? ad[8 * k + 2] : 0.0;
+        bq[k] = sg * (cs == 0 ? a : d);
+        bz[k] = kn[k] * (cs == 0 ? d : a);
+      }
+#pragma unroll
+      for (int m = 0; m < kCluTiles; m++) {
+        if (m < mt) {
+          const int g = 8 * m + (lane >> 2);
+          const double *z = Zs + g * kZs + (lane & 3);
+          double2 Q = make_double2(0.0, 0.0), Z = Q;
+#pragma unroll
+          for (int k = 0; k < KS; k++)
+            if (k < ks) {
+              const double zf = z[4 * k];
+              dmma(Q, zf, bq[k]);
+              dmma(Z, zf, bz[k]);
+            }
+          double2 x = make_double2(0.0, 0.0);  // and 0 past the last row
+          if (wid < nt4) x = XYs[(4 * wid + (lane & 3)) * ns + g];
+          const double a = x.x * Q.x - x.y * Q.y;
+          double ex = gl * a, ey = gmm * a, ez = x.x * Z.x - x.y * Z.y;
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) {
+            ex += __shfl_xor_sync(0xffffffffu, ex, o);
+            ey += __shfl_xor_sync(0xffffffffu, ey, o);
+            ez += __shfl_xor_sync(0xffffffffu, ez, o);
+          }
+          if ((lane & 3) == 0) {
+            part[wid][0][g] = ex;
+            part[wid][1][g] = ey;
+            part[wid][2][g] = ez;
+          }
+        }
+      }
+    }
+    if (it > 1 && wid == kCluWarps - 1) {  // the change of the last update
+      double v = lane < kCluMax * mt ? slot[32 * (it & 1) + lane] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      chg = v;
+      if (lane == 0) *more = v > A.thr && it < A.maxit;
+    }
+    __syncthreads();
+    if (it > 1 && !*more) break;
+    double c = 0.0;
+    if (upd) {
+      double p[kCluWarps];
+#pragma unroll
+      for (int u = 0; u < kCluWarps; u++) p[u] = part[u][uc][ug];
+#pragma unroll
+      for (int o = kCluWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < o; u++) p[u] += p[u + o];
+      double *at = reinterpret_cast<double *>(mu + uw) + uc;
+      const double Et = (eim[4 * ug + uc] + p[0]) + e0, m = polr * Et, d = *at - m;
+#pragma unroll
+      for (int b = 0; b < kCluMax; b++) *cl.map_shared_rank(at, b) = m;
+      c = d * d;
+      e_up = -0.5 * polr * (Et * e0);
+    }
+    it++;
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    if (wid < mt) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+      // read after the next step's first barrier, which orders it; by parity, since a slow
+      // block may still be reading the previous step's
+      if (lane < kCluMax) *cl.map_shared_rank(slot + 32 * (it & 1) + me * mt + wid, lane) = c;
+    }
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // the new dipoles are here
+  }
+  if (it > 1) {  // the last update's sums: the change is warp kCluWarps - 1's
+    if (wid < mt) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) e_up += __shfl_xor_sync(0xffffffffu, e_up, o);
+      if (lane == 0) *cl.map_shared_rank(slot + 64 + me * mt + wid, 0) = e_up;
+    }
+    cl.sync();
+  }
+  for (int u = tid; u < nloc * 3; u += kCluThreads) {
+    const double4 m = mu[w0 + u / 3];
+    A.mu[(size_t)w0 * 3 + u] = u % 3 == 0 ? m.x : (u % 3 == 1 ? m.y : m.z);
+  }
+  if (me == 0 && tid == kCluThreads - 32) {
+    if (it > 1) {
+      ene = 0.0;
+      for (int u = 0; u < kCluMax * mt; u++) ene += slot[64 + u];
+    }
+    A.state[kIterIters] = (double)it;
+    A.state[kIterChange] = chg;
+    A.state[kIterEnergy] = ene;
+    A.state[kIterFinished] = 1.0;
+  }
+}
+
 // The first Jacobi step from mu = 0 (nb_induction_model.f90:1317-1359), where T.mu and the
 // reciprocal field are zero: mu = alpha E0, with the change and energy sums the full step
 // forms, in one block.  It records iteration 1 in the state and, inside the graph, sets the
@@ -983,6 +1331,66 @@ cudaError_t launch_dip_first(const IterArgs &A, cudaStream_t st) {
 cudaError_t launch_pcg_first(const IterArgs &A, cudaStream_t st) {
   k_pcg_first<<<1, kFirstThreads, 0, st>>>(A);
   return cudaGetLastError();
+}
+
+namespace {
+template <int J>
+void clu_config(const IterArgs &A, cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at) {
+  cfg.gridDim = dim3(kCluMax);
+  cfg.blockDim = dim3(kCluThreads);
+  cfg.dynamicSmemBytes = sizeof(double) * CluSmem(J, A.nw, A.nrow).total;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kCluMax;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+template <int J>
+bool clu_fits(const IterArgs &A) {
+  // a block per (row tile, n tile), a warp per tile of four rows
+  if (clu_sites(A.nw) > 8 * kCluTiles || (A.nrow + 7) / 8 * J > kCluMax || A.nrow > 4 * kCluWarps ||
+      sizeof(double) * CluSmem(J, A.nw, A.nrow).total > kCluSmem)
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  clu_config<J>(A, cfg, at);
+  int n = 0;
+  const auto k = k_dip_cluster<J>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCluSmem) ==
+          cudaSuccess &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0)
+    return true;
+  (void)cudaGetLastError();  // no such cluster on this device: the step kernels run
+  return false;
+}
+template <int J>
+cudaError_t launch_clu_t(const IterArgs &A, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  clu_config<J>(A, cfg, at);
+  cfg.stream = st;
+  return cudaLaunchKernelEx(&cfg, k_dip_cluster<J>, A);
+}
+}  // namespace
+
+bool dip_cluster_fits(const IterArgs &A) {
+  if (!A.rows || A.cu || A.nw < 1 || A.nw > 8 * kCluTiles * kCluMax) return false;
+  switch (iter_row_tiles(A.nmax)) {
+    case 1: return clu_fits<1>(A);
+    case 2: return clu_fits<2>(A);
+    case 3: return clu_fits<3>(A);
+    default: return false;
+  }
+}
+
+cudaError_t launch_dip_cluster(const IterArgs &A, cudaStream_t st) {
+  switch (iter_row_tiles(A.nmax)) {
+    case 1: return launch_clu_t<1>(A, st);
+    case 2: return launch_clu_t<2>(A, st);
+    case 3: return launch_clu_t<3>(A, st);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_phase_factors(const double2 *tab, int nm, SiteSets S, int kl, int km, int kn,
