@@ -113,6 +113,8 @@ struct ccp_context {
   // the rows of the k-vector list by decreasing length (KRow) and 2 pi n / L by n, for the
   // row form of the dipole step
   KRow *d_rows = nullptr;
+  double2 *d_krw = nullptr;  // the row form's gather weights (k_krows.cu)
+  size_t krw_cap = 0;
   double *d_rn = nullptr;
   int nrow = 0, nrow_cap = 0, nrn_cap = 0;
   double kv_box = -1, kv_alpha = -1;
@@ -254,6 +256,7 @@ void free_ctx(ccp_context *c) {
   if (c->d_P) cudaFree(c->d_P);
   if (c->d_PM) cudaFree(c->d_PM);
   if (c->d_rows) cudaFree(c->d_rows);
+  if (c->d_krw) cudaFree(c->d_krw);
   if (c->d_rn) cudaFree(c->d_rn);
   if (c->h_istate) cudaFreeHost(c->h_istate);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
@@ -455,6 +458,14 @@ int ensure_kspace(ccp_context *c, double box) {
       c->nrn_cap = 0;
       CK(dalloc(&c->d_rn, (size_t)nz));
       c->nrn_cap = nz;
+    }
+    const size_t nw = iter_rows_fit(c->kmax[2]) ? krow_weight_len(c->nrow, c->kmax[2]) : 0;
+    if (nw > c->krw_cap) {
+      if (c->d_krw) cudaFree(c->d_krw);
+      c->d_krw = nullptr;
+      c->krw_cap = 0;
+      CK(dalloc(&c->d_krw, nw));
+      c->krw_cap = nw;
     }
     if (c->nrow)
       CK(cudaMemcpyAsync(c->d_rows, rows.data(), sizeof(KRow) * c->nrow, cudaMemcpyHostToDevice,
@@ -975,14 +986,24 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
     if (mask & (T_KSPACE | T_INDUCTION))
       LK(launch_ktab(c->d_com, c->d_act, nm, S, box, c->kmax[0], c->kmax[1], c->kmax[2], c->d_tab,
                      sk));
-    if (mask & T_KSPACE)
+    // the reciprocal sums by k-vector rows where the row form applies (k_krows.cu)
+    const bool krows = c->opt_rows && c->nk > 0 && iter_rows_fit(c->kmax[2]);
+    const KRowArgs KR = {c->d_kv, c->d_rows, c->nrow, c->d_rn, c->d_tab, nm, c->kmax[0],
+                         c->kmax[1], c->kmax[2], S, c->d_sk, c->d_krw};
+    if (krows && (mask & (T_KSPACE | T_INDUCTION))) {
+      CK(cudaMemsetAsync(c->d_sk, 0, sizeof(double) * 4 * (size_t)c->nk, sk));
+      LK(launch_krow_sums(false, KR, nullptr, sk));
+      LK(launch_krow_weights(false, KR, c->alpha, mask & T_KSPACE ? 1 : 0, c->d_scal, sk));
+      if (!(mask & T_INDUCTION)) LK(launch_krow_gather(false, KR, 0, nullptr, nullptr, fk, sk));
+    } else if (mask & T_KSPACE) {
       LK(launch_kspace_sums(0, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1], c->kmax[2],
                             c->d_mu, c->d_sk, sk));
+    }
     // the Ewald energy and forces from those sums: here when the chain is serial, or after
     // the dipole loop's inputs on the reciprocal branch's stream, beside the loop (which uses
-    // its own S(k) buffers)
-    const bool ewald_late = kfork && (mask & T_INDUCTION);
-    if ((mask & T_KSPACE) && !ewald_late) {
+    // its own S(k) buffers); by rows one gather gives the static field and the Ewald forces
+    const bool ewald_late = kfork && (mask & T_INDUCTION) && !krows;
+    if ((mask & T_KSPACE) && !ewald_late && !krows) {
       LK(launch_kspace_energy(0, c->d_kv, c->nk, c->d_sk, c->alpha, c->d_scal, sk));
       LK(launch_kspace_gather(0, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
                               c->kmax[2], c->d_mu, c->d_sk, nullptr, fk, sk));
@@ -992,11 +1013,16 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       pbeg(3, sm);
       // the static field's structure factors (charges, mode 1) are the Ewald sums' (mode 0):
       // when those ran, d_sk still holds them
-      if (!(mask & T_KSPACE))
-        LK(launch_kspace_sums(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
-                              c->kmax[2], c->d_mu, c->d_sk, sk));
-      LK(launch_kspace_gather(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
-                              c->kmax[2], c->d_mu, c->d_sk, c->d_e0k, fk, sk));
+      if (krows) {
+        const bool ew = mask & T_KSPACE;
+        LK(launch_krow_gather(false, KR, ew ? 0 : 1, nullptr, c->d_e0k, ew ? fk : nullptr, sk));
+      } else {
+        if (!(mask & T_KSPACE))
+          LK(launch_kspace_sums(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
+                                c->kmax[2], c->d_mu, c->d_sk, sk));
+        LK(launch_kspace_gather(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
+                                c->kmax[2], c->d_mu, c->d_sk, c->d_e0k, fk, sk));
+      }
       if (c->use_rows) {
         double2 *Zc = c->d_P + (size_t)((c->nrow + 7) / 8 * 8) * nm * S.np;
         LK(launch_phase_rows(c->d_tab, nm, S, c->kmax[0], c->kmax[1], c->kmax[2], c->d_rows,
@@ -1035,11 +1061,17 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       }
       LK(launch_pair_indforce(px, py, pz, pxs, pys, pzs, ld, c->d_act, c->d_nbr, c->d_nbrv,
                               c->d_ncnt, c->cap, nm, S, P, c->d_mu, c->d_f, c->d_scal, sm));
-      LK(launch_kspace_sums(3, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1], c->kmax[2],
-                            c->d_mu, c->d_sk, sk));
-      LK(launch_kspace_energy(3, c->d_kv, c->nk, c->d_sk, c->alpha, c->d_scal, sk));
-      LK(launch_kspace_gather(3, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
-                              c->kmax[2], c->d_mu, c->d_sk, nullptr, fk, sk));
+      if (krows) {  // d_sk still holds the charges' sums
+        LK(launch_krow_sums(true, KR, c->d_mu, sk));
+        LK(launch_krow_weights(true, KR, c->alpha, 1, c->d_scal, sk));
+        LK(launch_krow_gather(true, KR, 0, c->d_mu, nullptr, fk, sk));
+      } else {
+        LK(launch_kspace_sums(3, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
+                              c->kmax[2], c->d_mu, c->d_sk, sk));
+        LK(launch_kspace_energy(3, c->d_kv, c->nk, c->d_sk, c->alpha, c->d_scal, sk));
+        LK(launch_kspace_gather(3, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
+                                c->kmax[2], c->d_mu, c->d_sk, nullptr, fk, sk));
+      }
       if (kfork) {
         CK(cudaEventRecord(c->ev_k2, sk));
         CK(cudaStreamWaitEvent(sm, c->ev_k2, 0));

@@ -358,6 +358,28 @@ cudaError_t launch_ktab(const double4 *com, const double4 *act, int nm, SiteSets
 // energy: per-k energy/virial of modes 0 and 3 into scal;
 // gather: MODES 1, 2 write the field into out (zeroed by the launcher), 0 and 3 add forces
 // into f.
+// The same sums by rows of the k-vector list (k_krows.cu; n_max up to the row form's, see
+// iter_rows_fit): sums of the charges into sk[k][0..1] (cleared by the caller) or of the dipoles
+// into sk[k][2..3]; the gathers' weights from them, with the energy and virial if asked for; and
+// the gathers, of the charges' field (into e0k and, times the charge, into f; either may be null;
+// pol: polarisable sites only) or of the induction forces.
+struct KRowArgs {
+  const KVec *kv;
+  const KRow *rows;
+  int nrow;
+  const double *rn;  // rn[n + kn] = 2 pi n / L
+  const double2 *tab;
+  int nm, kl, km, kn;
+  SiteSets S;
+  double *sk;
+  double2 *w;  // krow_weight_len(nrow, kn) elements
+};
+size_t krow_weight_len(int nrow, int kn);
+cudaError_t launch_krow_sums(bool dip, const KRowArgs &A, const double *mu, cudaStream_t st);
+cudaError_t launch_krow_weights(bool ind, const KRowArgs &A, double alpha, int energy, double *scal,
+                                cudaStream_t st);
+cudaError_t launch_krow_gather(bool ind, const KRowArgs &A, int pol, const double *mu, double *e0k,
+                               double *f, cudaStream_t st);
 cudaError_t launch_kspace_sums(int mode, const KVec *kv, int nk, const double2 *tab, int nm,
                                SiteSets S, int kl, int km, int kn, const double *mu,
                                double *sk, cudaStream_t st);

@@ -1,7 +1,7 @@
 // ccp_kspace_fixed.cu -- reciprocal-space Ewald sum (kspace_ewald, ewald.f90:754-1173) for
 // callers that cannot let the library allocate device memory.
 //
-// Same kernels as the context form (k_kspace.cu, modes 0), but every temporary -- k-vector
+// Same kernels as the context form (k_krows.cu, k_kspace.cu mode 0), but every temporary -- k-vector
 // list, structure factors, per-site phase tables, packed positions, compact forces and the
 // energy accumulators -- is carved out of one file-scope device array of fixed size
 // (kFixedScratchBytes).  The entry point allocates no device or host memory on its success
@@ -53,35 +53,93 @@ int count_kvecs(int lmax, int mmax, int nmax) {
   return nk;
 }
 
-// One block writes the ordered k-vector list: each thread takes a contiguous run of the
-// lexicographic (l, m, n) candidates, and a block-wide exclusive scan of the kept counts
-// gives each run its output offset.
-__global__ void __launch_bounds__(1024)
-    k_fixed_kvecs(int lmax, int mmax, int nmax, double alp, double box, KVec *kv) {
-  __shared__ int scan[1024];
-  const int M = 2 * mmax + 1, N = 2 * nmax + 1;
-  const int total = (lmax + 1) * M * N;
+int count_rows(int lmax, int mmax, int nmax) {
+  const int klm = std::min(lmax, std::min(mmax, nmax));
+  int n = 0;
+  for (int l = 0; l <= lmax; l++)
+    for (int m = -mmax; m <= mmax; m++)
+      n += (l > 0 || m >= 0) && l * l + m * m + (l == 0 && m == 0) <= klm * klm;
+  return n;
+}
+
+// Block 0 writes the ordered k-vector list and, with `rows`, its rows (one per (l, m), KRow) and
+// the z components rn[n + nmax]: a thread counts the k-vectors and rows of a run of (l, m), an
+// exclusive scan gives the runs their places, and then the block's threads take the (l, m, n)
+// candidates in turn.  The other blocks pack molecule centres and charged-site offsets and clear
+// the compact forces, the energy/virial accumulators and the structure factors (all summed into
+// with atomics).
+constexpr int kSetupThreads = 1024, kMaxK = 64;
+__global__ void __launch_bounds__(kSetupThreads)
+    k_fixed_setup(int lmax, int mmax, int nmax, double alp, double box, KVec *kv, KRow *rows,
+                  double *rn, int nk, const double *__restrict__ x, const double *__restrict__ y,
+                  const double *__restrict__ z, const double *__restrict__ xs,
+                  const double *__restrict__ ys, const double *__restrict__ zs, int nm, int ld,
+                  SiteSets S, double4 *com, double4 *act, double *f, double *sk, double *scal) {
+  if (blockIdx.x > 0) {
+    const int t = (blockIdx.x - 1) * blockDim.x + threadIdx.x, stride = (gridDim.x - 1) * blockDim.x;
+    const int n = nm * S.nq;
+    if (t < nm) com[t] = make_double4(x[t], y[t], z[t], 0.0);
+    if (t < n) {
+      const int i = t / S.nq, r = t % S.nq;
+      const size_t o = (size_t)i * ld + S.qsite[r];
+      act[t] = make_double4(xs[o], ys[o], zs[o], S.q[r]);
+      f[t] = 0.0;
+      f[(size_t)n + t] = 0.0;
+      f[2 * (size_t)n + t] = 0.0;
+    }
+    if (t < S_COUNT) scal[t] = 0.0;
+    for (int u = t; u < 4 * nk; u += stride) sk[u] = 0.0;
+    return;
+  }
+  __shared__ int2 scan[kSetupThreads];
+  __shared__ int first[(kMaxK + 1) * (2 * kMaxK + 1)];  // of each (l, m), in the list
+  const int M = 2 * mmax + 1, N = 2 * nmax + 1, nlm = (lmax + 1) * M;
   const int klm = min(lmax, min(mmax, nmax)), klmsq = klm * klm;
-  const int per = (total + blockDim.x - 1) / blockDim.x;
-  const int c0 = min(total, (int)threadIdx.x * per), c1 = min(total, c0 + per);
-  int kept = 0;
+  const double twopi = 2.0 * ccpd::kPi, volmi = box * box * box;
+  auto reach = [&](int l, int m) {  // the largest n of (l, m), -1 for none
+    const int left = klmsq - l * l - m * m;
+    if (left < 0 || (l == 0 && m < 0)) return -1;
+    int n = (int)sqrtf((float)left);
+    while (n * n > left) n--;
+    while ((n + 1) * (n + 1) <= left) n++;
+    return l == 0 && m == 0 && n < 1 ? -1 : n;
+  };
+  const int per = (nlm + blockDim.x - 1) / blockDim.x;
+  const int c0 = min(nlm, (int)threadIdx.x * per), c1 = min(nlm, c0 + per);
+  int2 kept = make_int2(0, 0);
   for (int c = c0; c < c1; c++) {
-    const int l = c / (M * N), m = (c / N) % M - mmax, n = c % N - nmax;
-    kept += kvec_kept(l, m, n, klmsq);
+    const int l = c / M, m = c % M - mmax, n = reach(l, m);
+    kept.x += n < 0 ? 0 : (l == 0 && m == 0 ? n : 2 * n + 1);
+    kept.y += n >= 0;
   }
   scan[threadIdx.x] = kept;
   __syncthreads();
   for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-    const int v = threadIdx.x >= (unsigned)off ? scan[threadIdx.x - off] : 0;
+    const int2 v = threadIdx.x >= (unsigned)off ? scan[threadIdx.x - off] : make_int2(0, 0);
     __syncthreads();
-    scan[threadIdx.x] += v;
+    scan[threadIdx.x].x += v.x;
+    scan[threadIdx.x].y += v.y;
     __syncthreads();
   }
-  int o = scan[threadIdx.x] - kept;
-  const double twopi = 2.0 * ccpd::kPi, volmi = box * box * box;
+  int2 o = scan[threadIdx.x];
+  o.x -= kept.x;
+  o.y -= kept.y;
   for (int c = c0; c < c1; c++) {
-    const int l = c / (M * N), m = (c / N) % M - mmax, n = c % N - nmax;
+    const int l = c / M, m = c % M - mmax, n = reach(l, m);
+    first[c] = o.x;
+    if (n < 0) continue;
+    const int nlo = l == 0 && m == 0 ? 1 : -n, len = n - nlo + 1;
+    if (rows) rows[o.y] = {twopi * l / box, twopi * m / box, o.x, len, nlo, c};
+    o.x += len;
+    o.y++;
+  }
+  if (rows)
+    for (int n = threadIdx.x; n < N; n += blockDim.x) rn[n] = twopi * (n - nmax) / box;
+  __syncthreads();
+  for (int c = threadIdx.x; c < nlm * N; c += blockDim.x) {
+    const int lm = c / N, l = lm / M, m = lm - l * M - mmax, n = c - lm * N - nmax;
     if (!kvec_kept(l, m, n, klmsq)) continue;
+    const int nlo = l == 0 && m == 0 ? 1 : -reach(l, m);
     KVec k;
     k.rl = twopi * l / box;
     k.rm = twopi * m / box;
@@ -92,29 +150,8 @@ __global__ void __launch_bounds__(1024)
     k.m = m;
     k.n = n;
     k.pad = 0;
-    kv[o++] = k;
+    kv[first[lm] + n - nlo] = k;
   }
-}
-
-// Packs molecule centres and charged-site offsets, and clears the compact forces and the
-// energy/virial accumulators (both are summed into with atomics).
-__global__ void k_fixed_prep(const double *__restrict__ x, const double *__restrict__ y,
-                             const double *__restrict__ z, const double *__restrict__ xs,
-                             const double *__restrict__ ys, const double *__restrict__ zs, int nm,
-                             int ld, SiteSets S, double4 *com, double4 *act, double *f,
-                             double *scal) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = nm * S.nq;
-  if (t < nm) com[t] = make_double4(x[t], y[t], z[t], 0.0);
-  if (t < n) {
-    const int i = t / S.nq, r = t % S.nq;
-    const size_t o = (size_t)i * ld + S.qsite[r];
-    act[t] = make_double4(xs[o], ys[o], zs[o], S.q[r]);
-    f[t] = 0.0;
-    f[(size_t)n + t] = 0.0;
-    f[2 * (size_t)n + t] = 0.0;
-  }
-  if (t < S_COUNT) scal[t] = 0.0;
 }
 
 // Adds the compact charged-site forces into the caller's (molecule, ld) arrays and writes
@@ -156,7 +193,7 @@ extern "C" int ccp_kspace_ewald_fixed(const ccp_model *m, int nm, const double *
   if (nm < 1 || ld < m->ns) return fail(CCP_ERR_BAD_INPUT, "need nm >= 1 and ld >= sites per molecule");
   if (lmax < 1 || mmax < 1 || nmax < 1) return fail(CCP_ERR_BAD_INPUT, "k-max must be >= 1");
   if (!(box > 0.0) || !(alp > 0.0)) return fail(CCP_ERR_BAD_INPUT, "box and alpha must be > 0");
-  if (lmax > 64 || mmax > 64 || nmax > 64) return fail(CCP_ERR_CAPACITY, "k-max above 64");
+  if (lmax > kMaxK || mmax > kMaxK || nmax > kMaxK) return fail(CCP_ERR_CAPACITY, "k-max above 64");
 
   // charged sites only: the compact site set (active slot = charged slot)
   SiteSets S;
@@ -188,6 +225,14 @@ extern "C" int ccp_kspace_ewald_fixed(const ccp_model *m, int nm, const double *
                                       std::to_string(nm) + " molecules and " + std::to_string(nk) +
                                       " k-vectors; the fixed scratch holds " +
                                       std::to_string(kFixedScratchBytes) + " bytes");
+
+  // by rows of the k-vector list (k_krows.cu) where the form applies and the scratch has room
+  // for its rows and weights
+  const int nrow = count_rows(lmax, mmax, nmax);
+  const size_t b_row = up256(sizeof(KRow) * (size_t)nrow);
+  const size_t b_rn = up256(sizeof(double) * (2 * (size_t)nmax + 1));
+  const size_t b_w = up256(sizeof(double2) * krow_weight_len(nrow, nmax));
+  const bool krows = iter_rows_fit(nmax) && need + b_row + b_rn + b_w <= kFixedScratchBytes;
 
   // The launch checks below read the thread's last CUDA error.  An error that earlier work of
   // the caller left pending would be reported as this call's own, so such a call is refused
@@ -221,18 +266,28 @@ extern "C" int ccp_kspace_ewald_fixed(const ccp_model *m, int nm, const double *
   double *scal = reinterpret_cast<double *>(base + b_kv + b_sk + b_com + b_act + b_tab + b_f);
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int nthr = (int)std::max(nq, (size_t)S_COUNT);  // nq >= nm
-  k_fixed_kvecs<<<1, 1024, 0, st>>>(lmax, mmax, nmax, alp, box, kv);
-  k_fixed_prep<<<(nthr + 255) / 256, 256, 0, st>>>(x, y, z, xs, ys, zs, nm, ld, S, com, act, f,
-                                                    scal);
+  KRow *rows = reinterpret_cast<KRow *>(base + need);
+  double *rn = reinterpret_cast<double *>(base + need + b_row);
+  double2 *w = reinterpret_cast<double2 *>(base + need + b_row + b_rn);
+  const size_t nthr = std::max(nq, (size_t)S_COUNT);  // nq >= nm
+  k_fixed_setup<<<1 + (unsigned)((nthr + kSetupThreads - 1) / kSetupThreads), kSetupThreads, 0, st>>>(
+      lmax, mmax, nmax, alp, box, kv, krows ? rows : nullptr, rn, nk, x, y, z, xs, ys, zs, nm, ld, S,
+      com, act, f, sk, scal);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(CCP_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = launch_ktab(com, act, nm, S, box, lmax, mmax, nmax, tab, st)) != cudaSuccess ||
-      (e = launch_kspace_sums(0, kv, nk, tab, nm, S, lmax, mmax, nmax, nullptr, sk, st)) !=
-          cudaSuccess ||
-      (e = launch_kspace_energy(0, kv, nk, sk, alp, scal, st)) != cudaSuccess ||
-      (e = launch_kspace_gather(0, kv, nk, tab, nm, S, lmax, mmax, nmax, nullptr, sk, nullptr, f,
-                                st)) != cudaSuccess)
-    return fail(CCP_ERR_CUDA, cudaGetErrorString(e));
+  e = launch_ktab(com, act, nm, S, box, lmax, mmax, nmax, tab, st);
+  if (krows) {
+    const KRowArgs R = {kv, rows, nrow, rn, tab, nm, lmax, mmax, nmax, S, sk, w};
+    if (e == cudaSuccess) e = launch_krow_sums(false, R, nullptr, st);
+    if (e == cudaSuccess) e = launch_krow_weights(false, R, alp, 1, scal, st);
+    if (e == cudaSuccess) e = launch_krow_gather(false, R, 0, nullptr, nullptr, f, st);
+  } else {
+    if (e == cudaSuccess)
+      e = launch_kspace_sums(0, kv, nk, tab, nm, S, lmax, mmax, nmax, nullptr, sk, st);
+    if (e == cudaSuccess) e = launch_kspace_energy(0, kv, nk, sk, alp, scal, st);
+    if (e == cudaSuccess)
+      e = launch_kspace_gather(0, kv, nk, tab, nm, S, lmax, mmax, nmax, nullptr, sk, nullptr, f, st);
+  }
+  if (e != cudaSuccess) return fail(CCP_ERR_CUDA, cudaGetErrorString(e));
   k_fixed_finish<<<(int)((nq + 255) / 256), 256, 0, st>>>(
       f, nm, ld, S, scal, fxs, fys, fzs, qkcpe, vir);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(CCP_ERR_CUDA, cudaGetErrorString(e));
