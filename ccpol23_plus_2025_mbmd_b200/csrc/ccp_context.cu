@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -175,6 +176,13 @@ struct ccp_context {
   unsigned *d_ticket = nullptr;  // last-block ticket of the fused update kernel
   std::array<int, 5> clu_key{};  // sizes that clu_fits was asked for
   bool clu_fits = false;         // the solve in one cluster applies to them
+  std::array<int, 6> grid_key{};  // sizes that grid_blocks was asked for
+  int grid_blocks = 0;           // blocks of the solve in one grid, 0 where it does not apply
+  int opt_grid = 1;              // the solve in one grid (k_dip_grid) where it applies
+  bool grid_failed = false;      // a wait in it ran out: the step kernels from then on
+  bool grid_active = false;      // the last solve ran in one grid
+  double *d_grid = nullptr;
+  size_t grid_cap = 0;
   int ind_per_iter = 0;          // kernels per Jacobi iteration of the last solve
   std::vector<long long> ind_key;
   // phase factors of the polarisable sites for the dipole iteration (k_iter.cu), when they
@@ -257,6 +265,7 @@ void free_ctx(ccp_context *c) {
   if (c->d_PM) cudaFree(c->d_PM);
   if (c->d_rows) cudaFree(c->d_rows);
   if (c->d_krw) cudaFree(c->d_krw);
+  if (c->d_grid) cudaFree(c->d_grid);
   if (c->d_rn) cudaFree(c->d_rn);
   if (c->h_istate) cudaFreeHost(c->h_istate);
   if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
@@ -690,6 +699,59 @@ bool dip_cluster(ccp_context *c, const IterArgs &A) {
   return c->clu_fits;
 }
 
+// The blocks of k_dip_grid wait for one another, so at most one such kernel may be under way on
+// a device: two whose blocks hold the SMs in part would wait for good.  An evaluation takes the
+// grid form only if the last one launched on its device, by any context, has finished (the
+// event), and never waits for it.
+struct GridTurn {
+  std::mutex mu;
+  cudaEvent_t done = nullptr;
+};
+constexpr int kMaxDevices = 64;
+GridTurn g_grid[kMaxDevices];
+
+// Launches the solve in one grid if it applies and its turn is free; *done tells.
+int try_dip_grid(ccp_context *c, const IterArgs &A, cudaStream_t st, bool *done) {
+  *done = false;
+  if (!c->opt_grid || c->grid_failed || c->device < 0 || c->device >= kMaxDevices) return CCP_OK;
+  const std::array<int, 6> key = {A.nw, A.nrow, A.nmax, A.rows != nullptr, A.cu != nullptr, A.cap};
+  if (key != c->grid_key) {
+    c->grid_blocks = dip_grid_blocks(A, c->nsm);
+    c->grid_key = key;
+  }
+  if (!c->grid_blocks) return CCP_OK;
+  const size_t need = dip_grid_scratch(A);
+  if (need > c->grid_cap) {
+    if (c->d_grid) cudaFree(c->d_grid);
+    c->d_grid = nullptr;
+    c->grid_cap = 0;
+    CK(dalloc(&c->d_grid, need));
+    c->grid_cap = need;
+  }
+  GridTurn &T = g_grid[c->device];
+  std::lock_guard<std::mutex> lock(T.mu);
+  if (!T.done) {
+    CK(cudaEventCreateWithFlags(&T.done, cudaEventDisableTiming));
+  } else {
+    const cudaError_t e = cudaEventQuery(T.done);
+    if (e == cudaErrorNotReady) {
+      (void)cudaGetLastError();
+      return CCP_OK;
+    }
+    CK(e);
+  }
+  const cudaError_t e = launch_dip_grid(A, c->grid_blocks, c->d_grid, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    c->grid_failed = true;
+    return CCP_OK;
+  }
+  CK(e);
+  CK(cudaEventRecord(T.done, st));
+  *done = true;
+  return CCP_OK;
+}
+
 // The whole Jacobi solve from mu = 0.  The state {iterations, change, energy} is copied to
 // h_istate; in the graph form the copy completes at the evaluation's final synchronisation.
 int run_dipole_loop(ccp_context *c, cudaStream_t st) {
@@ -697,12 +759,25 @@ int run_dipole_loop(ccp_context *c, cudaStream_t st) {
   const bool pcg = pcg_solver(c);
   c->pcg_active = pcg;
   if (pcg && !c->d_pcg) CK(dalloc(&c->d_pcg, 4 * (size_t)c->nm * c->S.np * 3));
+  c->grid_active = false;
   const IterArgs A1 = make_iter_args(c, 0, 0, 0);
   if (c->opt_graph && dip_cluster(c, A1)) {
     if (!cuda_ok(launch_dip_cluster(A1, st), "dipole solve")) return CCP_ERR_CUDA;
     CK(cudaMemcpyAsync(c->h_istate, c->d_istate, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     c->ind_per_iter = 0;
     return CCP_OK;
+  }
+  if (c->opt_graph) {
+    bool done = false;
+    CK(cudaMemsetAsync(c->d_istate, 0, kIterStateLen * sizeof(double), st));
+    const int r = try_dip_grid(c, A1, st, &done);
+    if (r) return r;
+    if (done) {
+      CK(cudaMemcpyAsync(c->h_istate, c->d_istate, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
+      c->grid_active = true;
+      c->ind_per_iter = 0;
+      return CCP_OK;
+    }
   }
   const double thr = ind_threshold(c);
   CK(cudaMemsetAsync(c->d_istate, 0, kIterStateLen * sizeof(double), st));
@@ -1141,6 +1216,10 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       if (r) return r;
       continue;
     }
+    if ((mask & T_INDUCTION) && c->grid_active && c->h_istate[3] < 0.0) {
+      c->grid_failed = true;  // a wait ran out (the GPU was held by other work): once more
+      continue;
+    }
     c->pgrad_valid = gfs3 != nullptr;
     if (mask & T_INDUCTION) {
       o.iters = (int)c->h_istate[0];
@@ -1511,7 +1590,7 @@ int ccp_context_create(const ccp_model *m, int nm, double box0, int device, int 
   if (cudaMalloc(&c->d_istate, kIterStateLen * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&c->d_ticket, sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(c->d_ticket, 0, sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost((void **)&c->h_istate, 3 * sizeof(double)) != cudaSuccess)
+      cudaMallocHost((void **)&c->h_istate, 4 * sizeof(double)) != cudaSuccess)
     return fail("loop state");
   const size_t n = nm, nsi = (size_t)nm * m->ns, np3 = (size_t)nm * std::max(S.np, 1) * 3;
   bool ok = dalloc(&c->d_x, 3 * n) == cudaSuccess && dalloc(&c->d_com, n) == cudaSuccess &&
@@ -1672,7 +1751,9 @@ int ccp_context_set_timing(ccp_context *ctx, int on) {
 int ccp_context_set_option(ccp_context *ctx, const char *name, int value) {
   if (!ctx || !name) return CCP_ERR_BAD_INPUT;
   const std::string n(name);
-  if (n == "graph_loop") {
+  if (n == "dipole_grid") {
+    ctx->opt_grid = value != 0;
+  } else if (n == "graph_loop") {
     ctx->opt_graph = value != 0;
   } else if (n == "phase_matrix") {
     ctx->opt_phase = value != 0;
@@ -1764,6 +1845,10 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
     *value = ctx->opt_rows;
   } else if (n == "dipole_row_form_active") {
     *value = ctx->use_rows ? 1 : 0;
+  } else if (n == "dipole_grid") {
+    *value = ctx->opt_grid;
+  } else if (n == "dipole_grid_active") {
+    *value = ctx->grid_active;
   } else if (n == "dipole_cluster_active") {
     *value = ctx->opt_graph && ctx->clu_fits;
   } else if (n == "dipole_solver") {

@@ -30,6 +30,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ccp_device.cuh"
 
@@ -1259,6 +1260,512 @@ __global__ void __launch_bounds__(kCluThreads) k_dip_cluster(IterArgs A) {
   }
 }
 
+// ------------------------------------------------------------------ the solve in one grid
+// Middle sizes: the whole solve as one cooperative kernel, a block per SM that owns ns sites.
+// A step as two kernels costs 5 us per kernel before any work (launch, first loads, the
+// reduction's end), and beside the three-body kernels, whose blocks fill the SMs, each launch
+// also waits for its blocks' slots; here the blocks keep half of every SM for the solve, the
+// constant operands of a step are under way before the step begins, and a step has two grid
+// barriers.  Warps 0-3 of a block take (row tile, site chunk) units of the structure factors,
+// as k_iter_a_rows, warps 4-7 T.mu of the block's sites; after the barrier all gather the
+// block's sites over the rows, as k_iter_b_rows, and update them.  S(k) is kept as the
+// combinations that the gather takes, AD[row][n][(re), (im)] = (S(n) + S(-n), S(n) - S(-n)).
+// Data of other blocks is read past L1 (__ldcg).  A barrier's wait is bounded: a block that
+// waits longer marks the solve as failed and leaves, and the host takes the step kernels.
+constexpr int kGridThreads = 256, kGridWarps = kGridThreads / 32, kGridRowWarps = 4;
+constexpr int kGridSub = 16;     // sites that a row warp stages at a time
+constexpr int kGridStages = 4;  // stages of its ring, where a step's operands do not all stay
+constexpr int kGridEnt = 5;     // tensor entries that a lane has under way
+constexpr int kGridXs = 18;                    // doubles per staged site's XY (8 rows + padding)
+constexpr unsigned kGridSpins = 1u << 21;      // polls of a barrier, of about half a us each
+
+struct GridSmem {  // offsets in doubles
+  int v, ring, red, part, z, rn, eim, own, src, total, ns8;
+  __host__ __device__ GridSmem(int J, int nw, int ns, int ent, int stages) {
+    const int kz = 8 * J + 2;
+    ns8 = (ns + 7) / 8 * 8;
+    v = 0;                                                   // [nw + 64][3] the multiplied vector
+    ring = (3 * (nw + 64) + 1) / 2 * 2;                      // [warp][stage][16][kGridXs + kz]
+    red = ring + kGridRowWarps * stages * kGridSub * (kGridXs + kz);
+    part = red + kGridRowWarps * 4 * J * 64;                 // [warps][3][16]
+    z = part + kGridWarps * 3 * 16;                          // [ns8][kz]
+    rn = z + ns8 * kz;                                       // [4 J]
+    eim = rn + 4 * J;                                        // [ns][3]
+    own = eim + 3 * ns;                                      // [ns][3] reciprocal field
+    src = own + 3 * ns;                                      // 16 bits [ns][ent], then int [ns]
+    total = src + (ns * ent + 3) / 4 + (ns + 1) / 2;
+  }
+};
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// All blocks' writes before are visible to all blocks after; false when the wait ran out.
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    unsigned seen = 0, spins = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+    } while (seen < target && ++spins < kGridSpins);
+    *ok = seen >= target;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+template <bool PCG, int J>
+__global__ void __launch_bounds__(kGridThreads, 2) k_dip_grid(IterArgs A, GridArgs G) {
+  constexpr int KS = 2 * J, kZs = 8 * J + 2, kStage = kGridSub * (kGridXs + kZs), kN4 = 4 * J;
+  extern __shared__ double4 smu4[];
+  double *sm = reinterpret_cast<double *>(smu4);
+  __shared__ int ok;
+  const int ns = G.ns;
+  const int ent = A.cap * A.np;
+  const GridSmem L(J, A.nw, ns, ent, G.stages);
+  double *v = sm + L.v, *Zs = sm + L.z, *eim = sm + L.eim, *own = sm + L.own, *rn = sm + L.rn;
+  unsigned short *src = reinterpret_cast<unsigned short *>(sm + L.src);
+  int *n_ent = reinterpret_cast<int *>(sm + L.src + (ns * ent + 3) / 4);
+  __shared__ int ticket;
+  double2(*red)[4 * J][32] = reinterpret_cast<double2(*)[4 * J][32]>(sm + L.red);
+  double(*part)[3][16] = reinterpret_cast<double(*)[3][16]>(sm + L.part);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int w0 = blockIdx.x * ns, nloc = min(max(A.nw - w0, 0), ns);
+  const int nt8 = (A.nrow + 7) / 8, nt4 = (A.nrow + 3) / 4, nr8 = 8 * nt8;
+  const int n_unit = nt8 * G.nchunk;
+  const size_t ad_len = (size_t)nr8 * kN4 * 4;
+  unsigned target = 0;
+
+  for (int u = tid; u < L.ns8 * 4 * J; u += kGridThreads) {
+    const int g = u / (4 * J), c = u - g * (4 * J);
+    *reinterpret_cast<double2 *>(Zs + g * kZs + 2 * c) = reinterpret_cast<const double2 *>(
+        A.Zc + (size_t)min(w0 + g, A.nw - 1) * A.zs)[c];
+  }
+  for (int n = tid; n < 4 * J; n += kGridThreads) rn[n] = A.rn[min(n, A.nmax) + A.nmax];
+  for (int u = 3 * A.nw + tid; u < 3 * (A.nw + 64); u += kGridThreads) v[u] = 0.0;
+  for (int g = wid; g < nloc; g += kGridWarps) {  // source sites of the block's tensor entries
+    const int i = (w0 + g) / A.np, n = min(A.ncnt[i], A.cap) * A.np;
+    for (int e = lane; e < n; e += 32)
+      src[g * ent + e] = (unsigned short)(A.nbr[(size_t)i * A.cap + e / A.np] * A.np + e % A.np);
+    if (lane == 0) n_ent[g] = n;
+  }
+  // the block's sites at the start: the first Jacobi step (as k_dip_first), or PCG's zero
+  // iterate (as k_pcg_first)
+  {
+    double ch = 0.0, en = 0.0;
+    for (int u = tid; u < 3 * nloc; u += kGridThreads) {
+      const size_t o = (size_t)w0 * 3 + u;
+      const double e0 = A.e0[o], m = A.S.apol[(w0 + u / 3) % A.np] * e0;
+      if (PCG) {
+        A.mu[o] = A.cw[o] = A.cs[o] = A.cp[o] = 0.0;
+        A.cu[o] = m;
+      } else {
+        A.mu[o] = m;
+        ch += m * m;
+        en += -0.5 * m * e0;
+      }
+    }
+    if (!PCG) {
+      ch = warp_sum(ch);
+      en = warp_sum(en);
+      if (lane == 0 && 32 * wid < 3 * nloc) {
+        atomicAdd(&G.acc[4 + 0], ch);
+        atomicAdd(&G.acc[4 + 1], en);
+      }
+    }
+  }
+  // row warps: the constant operands of 16 sites (step sub of a unit) into a stage of the ring
+  double *ring = sm + L.ring + wid * G.stages * kStage;
+  auto fetch = [&](int unit, int sub, int stage) {
+    const int rt = unit / G.nchunk, s0 = (unit - rt * G.nchunk) * G.chunk + sub * 4 * kGridSub + wid * kGridSub;
+    double *d = ring + stage * kStage;
+    const double2 *xy = A.XYr + (size_t)rt * A.nw * 8;
+    for (int u = lane; u < kGridSub * 8; u += 32) {
+      const int w = min(s0 + (u >> 3), A.nw - 1);
+      cp_async16(d + (u >> 3) * kGridXs + 2 * (u & 7), xy + (size_t)w * 8 + (u & 7));
+    }
+    for (int u = lane; u < kGridSub * 4 * J; u += 32) {
+      const int q = u / (4 * J), c = u - q * (4 * J), w = min(s0 + q, A.nw - 1);
+      cp_async16(d + kGridSub * kGridXs + q * kZs + 2 * c, A.Zc + (size_t)w * A.zs + 2 * c);
+    }
+  };
+  const int subs = (G.chunk + 4 * kGridSub - 1) / (4 * kGridSub);
+  // what the ring takes next: the unit's next sites, the block's next unit and, as the tables
+  // stay, the next step's first
+  int next_unit = blockIdx.x, next_sub = 0, stage = 0;
+  auto fetch_next = [&](int st) {
+    fetch(next_unit, next_sub, st);
+    cp_async_commit();
+    if (++next_sub == subs) {
+      next_sub = 0;
+      next_unit += gridDim.x;
+      if (next_unit >= n_unit) next_unit = blockIdx.x;
+    }
+  };
+  if (wid < kGridRowWarps && (int)blockIdx.x < n_unit) {
+    for (int st = 0; st < G.stages; st++) fetch_next(st);
+    if (G.stay) cp_async_wait<0>();
+  }
+  double alpha = 0.0, beta = 0.0, gamma = 0.0, chg = 0.0, ene = 0.0;
+  int it = PCG ? 0 : 1;
+  bool more = !PCG || A.maxit >= 1;
+  const bool started = grid_barrier(G.bar, target += gridDim.x, &ok);
+  while (started && more) {
+    const int par = it & 1;
+    double *ad = G.ad + par * ad_len;
+    double chg_t = 0.0, ene_t = 0.0;
+    if (!PCG) {  // of the last update; the test is below, past the loads that follow
+      chg_t = __ldcg(&G.acc[4 * (it % 3)]);
+      ene_t = __ldcg(&G.acc[4 * (it % 3) + 1]);
+    }
+    // the whole vector
+    if (PCG) {
+      const int m3 = 3 * A.np, dc = kGridThreads % m3;
+      int c = tid % m3;  // component in the molecule
+#pragma unroll 6
+      for (int u = tid; u < 3 * A.nw; u += kGridThreads) {
+        v[u] = pcg_u(__ldcg(A.cu + u), pcg_s(__ldcg(A.cw + u), __ldcg(A.cs + u), beta),
+                     A.S.apol[c / 3], alpha);
+        c += dc;
+        if (c >= m3) c -= m3;
+      }
+    } else {
+      for (int u = tid; u < 3 * A.nw / 2; u += kGridThreads)
+        cp_async16(v + 2 * u, A.mu + 2 * u);
+      cp_async_commit();
+      if (tid == 0 && (A.nw & 1)) v[3 * A.nw - 1] = __ldcg(A.mu + 3 * A.nw - 1);
+    }
+    // the other parity's combinations, last read by the previous step's gather
+    for (size_t u = (size_t)blockIdx.x * kGridThreads + tid; u < ad_len / 2;
+         u += (size_t)gridDim.x * kGridThreads)
+      reinterpret_cast<double2 *>(G.ad + (par ^ 1) * ad_len)[u] = make_double2(0.0, 0.0);
+    if (blockIdx.x == 0 && tid < 4) G.acc[4 * ((it + 2) % 3) + tid] = 0.0;
+    if (tid == 0) ticket = 0;
+    if (!PCG) cp_async_wait<0>();
+    __syncthreads();
+    if (!PCG) {
+      chg = chg_t;
+      ene = ene_t;
+      if (!(chg > A.thr && it < A.maxit)) break;
+    }
+    if (wid < kGridRowWarps) {
+      for (int unit = blockIdx.x; unit < n_unit; unit += gridDim.x) {
+        const int rt = unit / G.nchunk, c0 = (unit - rt * G.nchunk) * G.chunk;
+        const int row = rt * 8 + (lane >> 2);
+        const KRow R = A.rows[min(row, A.nrow - 1)];
+        const int jt = warp_max(R.nlo + R.len - 1) / 4 + 1;
+        // kspace_efield_idm's weights (nb_induction_model.f90:2560-2600) of (row, n)
+        auto weights = [&](int n, double &gp, double &gm, double &kn) {
+          const int kp = n - R.nlo, km = -n - R.nlo;
+          gp = kp >= 0 && kp < R.len ? -4.0 * A.kv[R.kbeg + kp].ak : 0.0;
+          gm = n > 0 && km >= 0 && km < R.len ? -4.0 * A.kv[R.kbeg + km].ak : 0.0;
+          kn = A.rn[min(n, A.nmax) + A.nmax];
+        };
+        double gp0, gm0, kn0;  // the warp's n tile is wid (and 4 + wid)
+        weights(4 * wid + (lane & 3), gp0, gm0, kn0);
+        double2 acc[4][J];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+          for (int j = 0; j < J; j++) acc[c][j] = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int sub = 0; sub < subs; sub++) {
+          if (!G.stay) {
+            cp_async_wait<kGridStages - 1>();
+            __syncwarp();
+          }
+          const double *d = ring + stage * kStage, *xs = d + (lane & 3) * kGridXs + 2 * (lane >> 2),
+                       *zs = d + kGridSub * kGridXs + (lane & 3) * kZs + (lane >> 2);
+          const int q0 = sub * 4 * kGridSub + wid * kGridSub + (lane & 3);  // in the chunk
+          // by the row tile's n tiles: no branch between the products
+          auto run = [&](auto jc) {
+            constexpr int JT = decltype(jc)::value;
+#pragma unroll
+            for (int t = 0; t < kGridSub / 4; t++) {
+              const int q = q0 + 4 * t;
+              const double *m = v + 3 * (q < G.chunk ? min(c0 + q, A.nw) : A.nw);  // zeros past the end
+              const double2 xy = *reinterpret_cast<const double2 *>(xs + 4 * t * kGridXs);
+              const double dl = R.rl * m[0] + R.rm * m[1], mz = m[2];
+              const double a[4] = {xy.x * dl, xy.y * dl, xy.x * mz, xy.y * mz};
+#pragma unroll
+              for (int j = 0; j < JT; j++) {
+                const double z = zs[4 * t * kZs + 8 * j];
+#pragma unroll
+                for (int c = 0; c < 4; c++) dmma(acc[c][j], a[c], z);
+              }
+            }
+          };
+          if (J == 1 || jt == J) run(std::integral_constant<int, J>());
+          else if (J == 2 || jt == J - 1) run(std::integral_constant<int, (J > 1 ? J - 1 : 1)>());
+          else if (J == 3 || jt == J - 2) run(std::integral_constant<int, (J > 2 ? J - 2 : 1)>());
+          else run(std::integral_constant<int, (J > 3 ? J - 3 : 1)>());
+          if (!G.stay) {
+            __syncwarp();
+            fetch_next(stage);
+          }
+          if (++stage == G.stages) stage = 0;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+          for (int j = 0; j < J; j++) red[wid][c * J + j][lane] = acc[c][j];
+        asm volatile("bar.sync 1, %0;" ::"n"(kGridRowWarps * 32) : "memory");
+        for (int u = tid; u < jt * 32; u += kGridRowWarps * 32) {
+          const int j = u >> 5, n = 4 * j + (lane & 3);
+          if (row >= A.nrow || n > A.nmax) continue;
+          double2 s[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            double2 x[kGridRowWarps];
+#pragma unroll
+            for (int w = 0; w < kGridRowWarps; w++) x[w] = red[w][c * J + j][lane];
+            s[c].x = (x[0].x + x[1].x) + (x[2].x + x[3].x);
+            s[c].y = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+          }
+          double gp = gp0, gm = gm0, kn = kn0;
+          if (j != wid) weights(n, gp, gm, kn);
+          const double pr = gp * ((s[0].x - s[1].y) + kn * (s[2].x - s[3].y));
+          const double pi = gp * ((s[0].y + s[1].x) + kn * (s[2].y + s[3].x));
+          const double mr = gm * ((s[0].x + s[1].y) - kn * (s[2].x + s[3].y));
+          const double mi = gm * ((s[1].x - s[0].y) - kn * (s[3].x - s[2].y));
+          double *o = ad + ((size_t)row * kN4 + n) * 4;
+          atomicAdd(o, pr + mr);
+          atomicAdd(o + 1, pr - mr);
+          atomicAdd(o + 2, pi + mi);
+          atomicAdd(o + 3, pi - mi);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kGridRowWarps * 32) : "memory");
+      }
+    }
+    // T.mu of the block's sites, drawn by the warps one by one
+    for (;;) {
+      int g = 0;
+      if (lane == 0) g = atomicAdd(&ticket, 1);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (g >= nloc) break;
+      const int w = w0 + g, n = n_ent[g];
+      const double4 *T4 = A.T4 + (size_t)w * ent;
+      const double *TB = A.TB + (size_t)w * ent;
+      const unsigned short *sg = src + g * ent;
+      double ex = 0.0, ey = 0.0, ez = 0.0;
+      auto add = [&](const double4 &T, double B, const double *m) {
+        const double dm = T.w * (T.x * m[0] + T.y * m[1] + T.z * m[2]);
+        ex += dm * T.x - B * m[0];
+        ey += dm * T.y - B * m[1];
+        ez += dm * T.z - B * m[2];
+      };
+      if (lane < A.np)
+        add(A.S4[(size_t)w * A.np + lane], A.SB[(size_t)w * A.np + lane],
+            v + 3 * (w / A.np * A.np + lane));
+      for (int e0 = lane; e0 < n + lane; e0 += 32 * kGridEnt) {  // all lanes alike
+        double4 t[kGridEnt];
+        double b[kGridEnt];
+        int q[kGridEnt];
+#pragma unroll
+        for (int u = 0; u < kGridEnt; u++) {
+          const int e = e0 + 32 * u;
+          t[u] = make_double4(0.0, 0.0, 0.0, 0.0);
+          b[u] = 0.0;
+          q[u] = 0;
+          if (e < n) {
+            t[u] = T4[e];
+            b[u] = TB[e];
+            q[u] = sg[e];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kGridEnt; u++) add(t[u], b[u], v + 3 * q[u]);
+      }
+      ex = warp_sum(ex);
+      ey = warp_sum(ey);
+      ez = warp_sum(ez);
+      if (lane == 0) {
+        eim[3 * g] = ex;
+        eim[3 * g + 1] = ey;
+        eim[3 * g + 2] = ez;
+      }
+    }
+    if (!grid_barrier(G.bar, target += gridDim.x, &ok)) break;
+    // ---- gather, two tiles of 8 sites at a time
+    const int ri = (lane >> 2) & 1, cs = lane & 1, n0 = (lane >> 1) & 1, x = ri ^ cs;
+    const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
+    for (int g0 = 0; g0 < nloc; g0 += 16) {
+      const bool two = g0 + 8 < nloc;
+      const int wa = min(w0 + g0 + (lane >> 2), A.nw - 1), wb = min(w0 + g0 + 8 + (lane >> 2), A.nw - 1);
+      double e[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+      double2 f[KS], xa, xb;
+      double rl = 0.0, rm = 0.0;
+      int ks = 0;
+      auto load = [&](int t) {
+        const double2 *p = reinterpret_cast<const double2 *>(
+                               ad + ((size_t)(4 * t + (lane >> 3)) * kN4 + n0) * 4) + x;
+#pragma unroll
+        for (int k = 0; k < KS; k++) f[k] = __ldcg(p + 4 * k);
+        const KRow &Rb = A.rows[min(4 * t + (lane >> 3), A.nrow - 1)];
+        ks = Rb.nlo + Rb.len - 1;
+        const KRow &Ra = A.rows[min(4 * t + (lane & 3), A.nrow - 1)];
+        rl = Ra.rl;
+        rm = Ra.rm;
+        const double2 *xy = A.XYr + (size_t)(t >> 1) * A.nw * 8 + 4 * (t & 1) + (lane & 3);
+        xa = xy[(size_t)wa * 8];
+        xb = xy[(size_t)wb * 8];
+      };
+      if (wid < nt4) load(wid);
+      for (int t = wid; t < nt4; t += kGridWarps) {
+        const int kl = warp_max(ks) / 2 + 1;
+        double bq[KS], bz[KS];
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+          const double kn = rn[2 * k + n0];
+          bq[k] = sg * (cs == 0 ? f[k].x : f[k].y);
+          bz[k] = kn * (sg * (cs == 0 ? f[k].y : f[k].x));
+        }
+        const double2 ya = xa, yb = xb;
+        const double l = rl, m = rm;
+        if (t + kGridWarps < nt4) load(t + kGridWarps);
+        const double *za = Zs + (g0 + (lane >> 2)) * kZs + (lane & 3), *zb = za + 8 * kZs;
+        double2 Qa = make_double2(0.0, 0.0), Za = Qa, Qb = Qa, Zb = Qa;
+        auto run = [&](auto kc) {  // by two steps of n: no branch between the products
+          constexpr int KT = decltype(kc)::value;
+          if (two) {
+#pragma unroll
+            for (int k = 0; k < KT; k++) {
+              const double z = za[4 * k], z2 = zb[4 * k];
+              dmma(Qa, z, bq[k]);
+              dmma(Za, z, bz[k]);
+              dmma(Qb, z2, bq[k]);
+              dmma(Zb, z2, bz[k]);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < KT; k++) {
+              const double z = za[4 * k];
+              dmma(Qa, z, bq[k]);
+              dmma(Za, z, bz[k]);
+            }
+          }
+        };
+        if (J == 1 || kl > KS - 2) run(std::integral_constant<int, KS>());
+        else if (J == 2 || kl > KS - 4) run(std::integral_constant<int, (J > 1 ? KS - 2 : KS)>());
+        else if (J == 3 || kl > KS - 6) run(std::integral_constant<int, (J > 2 ? KS - 4 : KS)>());
+        else run(std::integral_constant<int, (J > 3 ? KS - 6 : KS)>());
+        const double a = ya.x * Qa.x - ya.y * Qa.y, b = yb.x * Qb.x - yb.y * Qb.y;
+        e[0][0] += l * a;
+        e[0][1] += m * a;
+        e[0][2] += ya.x * Za.x - ya.y * Za.y;
+        e[1][0] += l * b;
+        e[1][1] += m * b;
+        e[1][2] += yb.x * Zb.x - yb.y * Zb.y;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) e[h][c] += __shfl_xor_sync(0xffffffffu, e[h][c], o);
+          if ((lane & 3) == 0) part[wid][c][8 * h + (lane >> 2)] = e[h][c];
+        }
+      __syncthreads();
+      if (tid < 48) {
+        const int g = g0 + tid / 3, c = tid - tid / 3 * 3;
+        if (g < nloc) {
+          double s = 0.0;
+#pragma unroll
+          for (int u = 0; u < kGridWarps; u++) s += part[u][c][tid / 3];
+          own[3 * g + c] = s;
+        }
+      }
+      __syncthreads();
+    }
+    // ---- update of the block's sites, a thread per component
+    {
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      for (int u = tid; u < 3 * nloc; u += kGridThreads) {
+        const size_t o = (size_t)w0 * 3 + u;
+        const double ap = A.S.apol[(w0 + u / 3) % A.np], e0 = A.e0[o];
+        if (PCG) {  // the operations of pcg_update
+          const double u0 = A.cu[o], sn = pcg_s(A.cw[o], A.cs[o], beta);
+          const double p = __fma_rn(beta, A.cp[o], u0), xx = __fma_rn(alpha, p, A.mu[o]);
+          const double un = pcg_u(u0, sn, ap, alpha), wv = un / ap - (eim[u] + own[u]);
+          A.cs[o] = sn;
+          A.cp[o] = p;
+          A.mu[o] = xx;
+          A.cu[o] = un;
+          A.cw[o] = wv;
+          s0 += un * un / ap;
+          s1 += wv * un;
+          s2 += un * un;
+          s3 += -0.5 * xx * e0;
+        } else {
+          const double Et = (eim[u] + own[u]) + e0, m = ap * Et, d = v[o] - m;
+          A.mu[o] = m;
+          s0 += d * d;
+          s1 += -0.5 * ap * (Et * e0);
+        }
+      }
+      if (32 * wid < 3 * nloc) {
+        double *acc = G.acc + 4 * ((it + 1) % 3);
+        s0 = warp_sum(s0);
+        s1 = warp_sum(s1);
+        if (PCG) {
+          s2 = warp_sum(s2);
+          s3 = warp_sum(s3);
+        }
+        if (lane == 0) {
+          atomicAdd(acc, s0);
+          atomicAdd(acc + 1, s1);
+          if (PCG) {
+            atomicAdd(acc + 2, s2);
+            atomicAdd(acc + 3, s3);
+          }
+        }
+      }
+    }
+    it++;
+    if (!grid_barrier(G.bar, target += gridDim.x, &ok)) break;
+    if (PCG) {  // every block closes the step alike (pcg_update)
+      const double *acc = G.acc + 4 * (it % 3);
+      const double g1 = __ldcg(acc), d1 = __ldcg(acc + 1);
+      chg = __ldcg(acc + 2);
+      ene = __ldcg(acc + 3);
+      more = chg > A.thr && it < A.maxit;
+      if (more) {
+        const double b = it == 1 ? 0.0 : g1 / gamma;
+        const double a = it == 1 ? g1 / d1 : g1 / (d1 - b * g1 / alpha);
+        if (a > 0.0 && a < 1e300) {
+          alpha = a;
+          beta = b;
+          gamma = g1;
+        } else {  // breakdown (not positive definite): reported as no convergence
+          it = A.maxit;
+          more = false;
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+  if (tid == 0) {
+    if (!ok) {
+      A.state[kIterFinished] = -1.0;
+    } else if (blockIdx.x == 0) {
+      A.state[kIterIters] = (double)it;
+      A.state[kIterChange] = chg;
+      A.state[kIterEnergy] = ene;
+      A.state[kIterFinished] = 1.0;
+    }
+  }
+}
+
 // The first Jacobi step from mu = 0 (nb_induction_model.f90:1317-1359), where T.mu and the
 // reciprocal field are zero: mu = alpha E0, with the change and energy sums the full step
 // forms, in one block.  It records iteration 1 in the state and, inside the graph, sets the
@@ -1389,6 +1896,89 @@ cudaError_t launch_dip_cluster(const IterArgs &A, cudaStream_t st) {
     case 1: return launch_clu_t<1>(A, st);
     case 2: return launch_clu_t<2>(A, st);
     case 3: return launch_clu_t<3>(A, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+namespace {
+constexpr size_t kGridStay = 176 * 1024;
+template <bool PCG, int J>
+int grid_blocks_t(const IterArgs &A, int nsm) {
+  const int nb = std::min(nsm, (A.nw + 7) / 8), ns = (A.nw + nb - 1) / nb;
+  const size_t smem = sizeof(double) * GridSmem(J, A.nw, ns, A.cap * A.np, kGridStages).total;
+  const auto k = k_dip_grid<PCG, J>;
+  int per_sm = 0;
+  if (smem > kCluSmem || A.nw > 65535 ||  // 16-bit site numbers
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCluSmem) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGridThreads, smem) != cudaSuccess ||
+      per_sm < 1) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return (A.nw + ns - 1) / ns;
+}
+template <bool PCG, int J>
+cudaError_t launch_grid_t(const IterArgs &A, GridArgs G, int blocks, cudaStream_t st) {
+  // all operands of a block's one unit stay where they fit beside the rest
+  const int subs = G.chunk / (kGridRowWarps * kGridSub), ent = A.cap * A.np;
+  G.stay = (A.nrow + 7) / 8 * G.nchunk <= blocks &&
+           sizeof(double) * GridSmem(J, A.nw, G.ns, ent, subs).total <= kGridStay;
+  G.stages = G.stay ? subs : kGridStages;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kGridThreads);
+  cfg.dynamicSmemBytes = sizeof(double) * GridSmem(J, A.nw, G.ns, ent, G.stages).total;
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_dip_grid<PCG, J>, A, G);
+}
+}  // namespace
+
+int dip_grid_blocks(const IterArgs &A, int nsm) {
+  if (!A.rows || A.nrow < 1 || A.nw < 1) return 0;
+  switch (iter_row_tiles(A.nmax)) {
+    case 1: return A.cu ? grid_blocks_t<true, 1>(A, nsm) : grid_blocks_t<false, 1>(A, nsm);
+    case 2: return A.cu ? grid_blocks_t<true, 2>(A, nsm) : grid_blocks_t<false, 2>(A, nsm);
+    case 3: return A.cu ? grid_blocks_t<true, 3>(A, nsm) : grid_blocks_t<false, 3>(A, nsm);
+    case 4: return A.cu ? grid_blocks_t<true, 4>(A, nsm) : grid_blocks_t<false, 4>(A, nsm);
+    default: return 0;
+  }
+}
+
+size_t dip_grid_scratch(const IterArgs &A) {  // doubles: counter, sums, combinations
+  return 16 + 2 * (size_t)((A.nrow + 7) / 8 * 8) * 4 * iter_row_tiles(A.nmax) * 4;
+}
+
+cudaError_t launch_dip_grid(const IterArgs &A, int blocks, double *scratch, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(double) * dip_grid_scratch(A), st);
+  if (e != cudaSuccess) return e;
+  GridArgs G = {};
+  G.bar = reinterpret_cast<unsigned *>(scratch);
+  G.acc = scratch + 4;
+  G.ad = scratch + 16;
+  G.ns = (A.nw + blocks - 1) / blocks;
+  // sites per unit: the fewest steps of the busiest block, where a unit costs some six besides
+  const int nt8 = (A.nrow + 7) / 8, sub = kGridRowWarps * kGridSub, most = (A.nw + sub - 1) / sub;
+  long long best = -1;
+  for (int n = 1; n <= most; n++) {
+    const int nchunk = (most + n - 1) / n;
+    const long long cost = (long long)((nt8 * nchunk + blocks - 1) / blocks) * (n * (kGridSub / 4) + 6);
+    if (best < 0 || cost < best) {
+      best = cost;
+      G.chunk = n * sub;
+      G.nchunk = nchunk;
+    }
+  }
+  switch (iter_row_tiles(A.nmax)) {
+    case 1: return A.cu ? launch_grid_t<true, 1>(A, G, blocks, st) : launch_grid_t<false, 1>(A, G, blocks, st);
+    case 2: return A.cu ? launch_grid_t<true, 2>(A, G, blocks, st) : launch_grid_t<false, 2>(A, G, blocks, st);
+    case 3: return A.cu ? launch_grid_t<true, 3>(A, G, blocks, st) : launch_grid_t<false, 3>(A, G, blocks, st);
+    case 4: return A.cu ? launch_grid_t<true, 4>(A, G, blocks, st) : launch_grid_t<false, 4>(A, G, blocks, st);
     default: return cudaErrorInvalidValue;
   }
 }
