@@ -1065,11 +1065,13 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
     const bool krows = c->opt_rows && c->nk > 0 && iter_rows_fit(c->kmax[2]);
     const KRowArgs KR = {c->d_kv, c->d_rows, c->nrow, c->d_rn, c->d_tab, nm, c->kmax[0],
                          c->kmax[1], c->kmax[2], S, c->d_sk, c->d_krw};
+    const size_t nfs = (size_t)nm * ns;
+    const KRowForces KF = {fk, fk + nfs, fk + 2 * nfs, ns, nullptr, nullptr, nullptr};
     if (krows && (mask & (T_KSPACE | T_INDUCTION))) {
       CK(cudaMemsetAsync(c->d_sk, 0, sizeof(double) * 4 * (size_t)c->nk, sk));
       LK(launch_krow_sums(false, KR, nullptr, sk));
       LK(launch_krow_weights(false, KR, c->alpha, mask & T_KSPACE ? 1 : 0, c->d_scal, sk));
-      if (!(mask & T_INDUCTION)) LK(launch_krow_gather(false, KR, 0, nullptr, nullptr, fk, sk));
+      if (!(mask & T_INDUCTION)) LK(launch_krow_gather(false, KR, 0, nullptr, nullptr, KF, sk));
     } else if (mask & T_KSPACE) {
       LK(launch_kspace_sums(0, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1], c->kmax[2],
                             c->d_mu, c->d_sk, sk));
@@ -1090,7 +1092,7 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       // when those ran, d_sk still holds them
       if (krows) {
         const bool ew = mask & T_KSPACE;
-        LK(launch_krow_gather(false, KR, ew ? 0 : 1, nullptr, c->d_e0k, ew ? fk : nullptr, sk));
+        LK(launch_krow_gather(false, KR, ew ? 0 : 1, nullptr, c->d_e0k, ew ? KF : KRowForces{}, sk));
       } else {
         if (!(mask & T_KSPACE))
           LK(launch_kspace_sums(1, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
@@ -1139,7 +1141,7 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       if (krows) {  // d_sk still holds the charges' sums
         LK(launch_krow_sums(true, KR, c->d_mu, sk));
         LK(launch_krow_weights(true, KR, c->alpha, 1, c->d_scal, sk));
-        LK(launch_krow_gather(true, KR, 0, c->d_mu, nullptr, fk, sk));
+        LK(launch_krow_gather(true, KR, 0, c->d_mu, nullptr, KF, sk));
       } else {
         LK(launch_kspace_sums(3, c->d_kv, c->nk, c->d_tab, nm, S, c->kmax[0], c->kmax[1],
                               c->kmax[2], c->d_mu, c->d_sk, sk));

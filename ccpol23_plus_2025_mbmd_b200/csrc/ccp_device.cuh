@@ -375,7 +375,7 @@ cudaError_t launch_ktab(const double4 *com, const double4 *act, int nm, SiteSets
 // The same sums by rows of the k-vector list (k_krows.cu; n_max up to the row form's, see
 // iter_rows_fit): sums of the charges into sk[k][0..1] (cleared by the caller) or of the dipoles
 // into sk[k][2..3]; the gathers' weights from them, with the energy and virial if asked for; and
-// the gathers, of the charges' field (into e0k and, times the charge, into f; either may be null;
+// the gathers, of the charges' field (into e0k and, times the charge, into F; e0k, F.x may be null;
 // pol: polarisable sites only) or of the induction forces.
 struct KRowArgs {
   const KVec *kv;
@@ -392,8 +392,15 @@ size_t krow_weight_len(int nrow, int kn);
 cudaError_t launch_krow_sums(bool dip, const KRowArgs &A, const double *mu, cudaStream_t st);
 cudaError_t launch_krow_weights(bool ind, const KRowArgs &A, double alpha, int energy, double *scal,
                                 cudaStream_t st);
+struct KRowForces {  // added to: x[molecule * ld + site] and so on
+  double *x, *y, *z;
+  int ld;
+  // or null: the Ewald energy (kcal/mol, overwritten) and virial (added to), from scal
+  double *e, *vir;
+  const double *scal;
+};
 cudaError_t launch_krow_gather(bool ind, const KRowArgs &A, int pol, const double *mu, double *e0k,
-                               double *f, cudaStream_t st);
+                               const KRowForces &F, cudaStream_t st);
 cudaError_t launch_kspace_sums(int mode, const KVec *kv, int nk, const double2 *tab, int nm,
                                SiteSets S, int kl, int km, int kn, const double *mu,
                                double *sk, cudaStream_t st);

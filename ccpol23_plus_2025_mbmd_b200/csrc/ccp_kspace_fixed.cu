@@ -65,27 +65,34 @@ int count_rows(int lmax, int mmax, int nmax) {
 // Block 0 writes the ordered k-vector list and, with `rows`, its rows (one per (l, m), KRow) and
 // the z components rn[n + nmax]: a thread counts the k-vectors and rows of a run of (l, m), an
 // exclusive scan gives the runs their places, and then the block's threads take the (l, m, n)
-// candidates in turn.  The other blocks pack molecule centres and charged-site offsets and clear
-// the compact forces, the energy/virial accumulators and the structure factors (all summed into
-// with atomics).
-constexpr int kSetupThreads = 1024, kMaxK = 64;
+// candidates in turn.  The other blocks build the charged sites' phase tables (as k_ktab) and
+// clear the compact forces, the energy/virial accumulators and the structure factors (all summed
+// into with atomics).
+constexpr int kSetupThreads = 512, kMaxK = 64;
 __global__ void __launch_bounds__(kSetupThreads)
     k_fixed_setup(int lmax, int mmax, int nmax, double alp, double box, KVec *kv, KRow *rows,
                   double *rn, int nk, const double *__restrict__ x, const double *__restrict__ y,
                   const double *__restrict__ z, const double *__restrict__ xs,
                   const double *__restrict__ ys, const double *__restrict__ zs, int nm, int ld,
-                  SiteSets S, double4 *com, double4 *act, double *f, double *sk, double *scal) {
+                  SiteSets S, int k1, double2 *tab, double *f, double *sk, double *scal) {
   if (blockIdx.x > 0) {
     const int t = (blockIdx.x - 1) * blockDim.x + threadIdx.x, stride = (gridDim.x - 1) * blockDim.x;
     const int n = nm * S.nq;
-    if (t < nm) com[t] = make_double4(x[t], y[t], z[t], 0.0);
     if (t < n) {
       const int i = t / S.nq, r = t % S.nq;
       const size_t o = (size_t)i * ld + S.qsite[r];
-      act[t] = make_double4(xs[o], ys[o], zs[o], S.q[r]);
-      f[t] = 0.0;
-      f[(size_t)n + t] = 0.0;
-      f[2 * (size_t)n + t] = 0.0;
+      const double p[3] = {x[i] + xs[o], y[i] + ys[o], z[i] + zs[o]};
+      for (int a = 0; a < 3; a++) {
+        double2 *T = tab + (size_t)a * k1 * n + t;
+        double c1, s1;
+        sincos(2.0 * ccpd::kPi * p[a] / box, &s1, &c1);
+        double2 v = make_double2(1.0, 0.0);
+        for (int l = 0; l < k1; l++) {
+          T[(size_t)l * n] = v;
+          v = l == 0 ? make_double2(c1, s1) : make_double2(v.x * c1 - v.y * s1, v.y * c1 + v.x * s1);
+        }
+        f[(size_t)a * n + t] = 0.0;
+      }
     }
     if (t < S_COUNT) scal[t] = 0.0;
     for (int u = t; u < 4 * nk; u += stride) sk[u] = 0.0;
@@ -259,8 +266,6 @@ extern "C" int ccp_kspace_ewald_fixed(const ccp_model *m, int nm, const double *
   }
   KVec *kv = reinterpret_cast<KVec *>(base);
   double *sk = reinterpret_cast<double *>(base + b_kv);
-  double4 *com = reinterpret_cast<double4 *>(base + b_kv + b_sk);
-  double4 *act = reinterpret_cast<double4 *>(base + b_kv + b_sk + b_com);
   double2 *tab = reinterpret_cast<double2 *>(base + b_kv + b_sk + b_com + b_act);
   double *f = reinterpret_cast<double *>(base + b_kv + b_sk + b_com + b_act + b_tab);
   double *scal = reinterpret_cast<double *>(base + b_kv + b_sk + b_com + b_act + b_tab + b_f);
@@ -272,14 +277,17 @@ extern "C" int ccp_kspace_ewald_fixed(const ccp_model *m, int nm, const double *
   const size_t nthr = std::max(nq, (size_t)S_COUNT);  // nq >= nm
   k_fixed_setup<<<1 + (unsigned)((nthr + kSetupThreads - 1) / kSetupThreads), kSetupThreads, 0, st>>>(
       lmax, mmax, nmax, alp, box, kv, krows ? rows : nullptr, rn, nk, x, y, z, xs, ys, zs, nm, ld, S,
-      com, act, f, sk, scal);
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail(CCP_ERR_CUDA, cudaGetErrorString(e));
-  e = launch_ktab(com, act, nm, S, box, lmax, mmax, nmax, tab, st);
-  if (krows) {
-    const KRowArgs R = {kv, rows, nrow, rn, tab, nm, lmax, mmax, nmax, S, sk, w};
+      k1, tab, f, sk, scal);
+  e = cudaGetLastError();
+  if (krows) {  // the gather adds to the caller's forces
+    SiteSets Sr = S;
+    for (int r = 0; r < S.nq; r++) Sr.asite[r] = S.qsite[r];
+    const KRowArgs R = {kv, rows, nrow, rn, tab, nm, lmax, mmax, nmax, Sr, sk, w};
     if (e == cudaSuccess) e = launch_krow_sums(false, R, nullptr, st);
     if (e == cudaSuccess) e = launch_krow_weights(false, R, alp, 1, scal, st);
-    if (e == cudaSuccess) e = launch_krow_gather(false, R, 0, nullptr, nullptr, f, st);
+    if (e == cudaSuccess)
+      e = launch_krow_gather(false, R, 0, nullptr, nullptr, {fxs, fys, fzs, ld, qkcpe, vir, scal}, st);
+    return e == cudaSuccess ? CCP_OK : fail(CCP_ERR_CUDA, cudaGetErrorString(e));
   } else {
     if (e == cudaSuccess)
       e = launch_kspace_sums(0, kv, nk, tab, nm, S, lmax, mmax, nmax, nullptr, sk, st);

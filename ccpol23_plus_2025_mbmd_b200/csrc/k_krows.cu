@@ -211,13 +211,15 @@ __global__ void k_krow_weights(const KVec *__restrict__ kv, const KRow *__restri
 // Gathers: a block takes MT tiles of 8 sites, its warps the tiles of four rows in turn.  Lane l
 // ends up with the row sums of site l / 4 and row l % 4 and contracts them with XY.  Field form
 // (IND false): E into e0k of the polarisable sites (if set) and q E into the forces of the
-// charged ones (if f is set); sites: all active ones, or the polarisable ones only (pol).
+// charged ones (if F.x is set); sites: all active ones, or the polarisable ones only (pol).  With
+// F.e the field form also writes the Ewald energy (kcal/mol) and adds the virial, from the sums
+// that k_krow_weights left in scal, with the reference's prefactors (ewald.f90:1151-1160).
 template <bool IND, int J, int MT>
 __global__ void __launch_bounds__(kT)
     k_krow_gather(const KRow *__restrict__ rows, int nrow, const double2 *__restrict__ wt,
                   const double2 *__restrict__ tab, int nm, SiteSets S, int pol, int k1, int mmax,
                   int nmax, const double *__restrict__ rn, const double *__restrict__ mu,
-                  double *e0k, double *f) {
+                  double *e0k, KRowForces F) {
   constexpr int KS = 2 * J, kZs = 8 * J + 2, NS = 8 * MT, G = IND ? 4 : 2;
   extern __shared__ __align__(16) double4 smem4[];
   double2 *T = reinterpret_cast<double2 *>(smem4);        // [2 k1][NS]
@@ -339,7 +341,8 @@ __global__ void __launch_bounds__(kT)
 #pragma unroll
       for (int u = 0; u < kWarps; u++) v += part[u][c][s];
       const int st = slot(g), i = st / S.na, a = st - i * S.na;
-      const size_t o = (size_t)c * nm * S.ns + (size_t)i * S.ns + S.asite[a];
+      double *f = c == 0 ? F.x : (c == 1 ? F.y : F.z);
+      const size_t o = (size_t)i * F.ld + S.asite[a];
       if (IND) {
         atomicAdd(&f[o], kR4pie0 * v);
       } else {
@@ -347,6 +350,10 @@ __global__ void __launch_bounds__(kT)
         if (e0k && S.p_of_a[a] >= 0) e0k[((size_t)i * S.np + S.p_of_a[a]) * 3 + c] = v;
       }
     }
+  }
+  if (!IND && F.e && blockIdx.x == 0 && threadIdx.x == 0) {
+    *F.e = 2.0 * kR4pie0 * F.scal[S_KC_E] / 418.4;
+    *F.vir += 2.0 * kR4pie0 * F.scal[S_KC_VIR];
   }
 }
 
@@ -380,23 +387,23 @@ cudaError_t sums_t(const KRowArgs &A, const double *mu, cudaStream_t st) {
 }
 
 template <bool IND, int J, int MT>
-cudaError_t gather_mt(const KRowArgs &A, int pol, const double *mu, double *e0k, double *f,
+cudaError_t gather_mt(const KRowArgs &A, int pol, const double *mu, double *e0k, const KRowForces &F,
                       cudaStream_t st) {
   const int k1 = k1_of(A.kl, A.km, A.kn), total = A.nm * (pol ? A.S.np : A.S.na), NS = 8 * MT;
   const size_t smem = sizeof(double2) * 2 * k1 * NS + sizeof(double) * NS * (8 * J + 2);
   cudaError_t e = set_smem(k_krow_gather<IND, J, MT>, smem);
   if (e != cudaSuccess) return e;
   k_krow_gather<IND, J, MT><<<(total + NS - 1) / NS, kT, smem, st>>>(
-      A.rows, A.nrow, A.w, A.tab, A.nm, A.S, pol, k1, A.km, A.kn, A.rn, mu, e0k, f);
+      A.rows, A.nrow, A.w, A.tab, A.nm, A.S, pol, k1, A.km, A.kn, A.rn, mu, e0k, F);
   return cudaGetLastError();
 }
 template <bool IND, int J>
-cudaError_t gather_t(const KRowArgs &A, int pol, const double *mu, double *e0k, double *f,
+cudaError_t gather_t(const KRowArgs &A, int pol, const double *mu, double *e0k, const KRowForces &F,
                      cudaStream_t st) {
   // 16 sites per block once 8 make more than three waves: an operand then serves both tiles
   const int total = A.nm * (pol ? A.S.np : A.S.na);
-  return total > 8 * 148 * 6 ? gather_mt<IND, J, 2>(A, pol, mu, e0k, f, st)
-                             : gather_mt<IND, J, 1>(A, pol, mu, e0k, f, st);
+  return total > 8 * 148 * 6 ? gather_mt<IND, J, 2>(A, pol, mu, e0k, F, st)
+                             : gather_mt<IND, J, 1>(A, pol, mu, e0k, F, st);
 }
 
 }  // namespace
@@ -428,14 +435,14 @@ cudaError_t launch_krow_weights(bool ind, const KRowArgs &A, double alpha, int e
 }
 
 cudaError_t launch_krow_gather(bool ind, const KRowArgs &A, int pol, const double *mu, double *e0k,
-                               double *f, cudaStream_t st) {
+                               const KRowForces &F, cudaStream_t st) {
   if (A.nrow <= 0) return cudaSuccess;
   switch (iter_row_tiles(A.kn)) {
-    case 1: return ind ? gather_t<true, 1>(A, pol, mu, e0k, f, st) : gather_t<false, 1>(A, pol, mu, e0k, f, st);
-    case 2: return ind ? gather_t<true, 2>(A, pol, mu, e0k, f, st) : gather_t<false, 2>(A, pol, mu, e0k, f, st);
-    case 3: return ind ? gather_t<true, 3>(A, pol, mu, e0k, f, st) : gather_t<false, 3>(A, pol, mu, e0k, f, st);
-    case 4: return ind ? gather_t<true, 4>(A, pol, mu, e0k, f, st) : gather_t<false, 4>(A, pol, mu, e0k, f, st);
-    case 5: return ind ? gather_t<true, 5>(A, pol, mu, e0k, f, st) : gather_t<false, 5>(A, pol, mu, e0k, f, st);
+    case 1: return ind ? gather_t<true, 1>(A, pol, mu, e0k, F, st) : gather_t<false, 1>(A, pol, mu, e0k, F, st);
+    case 2: return ind ? gather_t<true, 2>(A, pol, mu, e0k, F, st) : gather_t<false, 2>(A, pol, mu, e0k, F, st);
+    case 3: return ind ? gather_t<true, 3>(A, pol, mu, e0k, F, st) : gather_t<false, 3>(A, pol, mu, e0k, F, st);
+    case 4: return ind ? gather_t<true, 4>(A, pol, mu, e0k, F, st) : gather_t<false, 4>(A, pol, mu, e0k, F, st);
+    case 5: return ind ? gather_t<true, 5>(A, pol, mu, e0k, F, st) : gather_t<false, 5>(A, pol, mu, e0k, F, st);
     default: return cudaErrorInvalidValue;
   }
 }
