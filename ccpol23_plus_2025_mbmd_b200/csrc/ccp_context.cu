@@ -145,6 +145,8 @@ struct ccp_context {
   bool have_vdw = false;
   int vdw_nrows = 0, vdw_nv = 0;
   int *d_vdw_row = nullptr, *d_vdw_site = nullptr;
+  int2 *d_vdw_spec = nullptr;  // site pairs with a charge product or dispersion
+  int vdw_nspec = 0;
   double *d_vdw_qq = nullptr, *d_vdw_par = nullptr;
   // FS3 parameters of this context (host copies): class coefficients, the class of every
   // coefficient-table entry, site-pair (b, g, r0); and the parameter-gradient buffer
@@ -244,7 +246,7 @@ void free_ctx(ccp_context *c) {
                 c->d_eik, c->d_eislf, c->d_eis, c->d_nbr,   c->d_ncnt, c->d_nbrv,  c->d_tri,
                 c->d_pairs, c->d_kv, c->d_kg, c->d_tab, c->d_sk, c->d_skj, c->d_coef, c->d_bgr,
                 c->d_types,
-                c->d_gfs3,  c->d_vdw_row, c->d_vdw_site, c->d_vdw_qq, c->d_vdw_par,
+                c->d_gfs3,  c->d_vdw_row, c->d_vdw_site, c->d_vdw_spec, c->d_vdw_qq, c->d_vdw_par,
                 c->d_pcoord, c->d_md_x, c->d_md_xs, c->d_md_v, c->d_md_q, c->d_md_j, c->d_md_red,
                 c->d_mu2, c->d_e0tot, c->d_eim, c->d_T4, c->d_S4, c->d_TB, c->d_SB,
                 c->d_pcg, c->d_cells, c->d_fpair};
@@ -1038,7 +1040,7 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       pbeg(9, s2);
       LK(launch_vdw(pxs, pys, pzs, ld, c->d_nbr, c->d_nbrv, c->d_ncnt, c->cap, nm, ns,
                     c->rcutsd, c->d_vdw_row, c->d_vdw_qq, c->d_vdw_par, c->vdw_nrows,
-                    c->d_vdw_site, c->vdw_nv, f3, c->d_scal, s2));
+                    c->d_vdw_site, c->vdw_nv, c->d_vdw_spec, c->vdw_nspec, f3, c->d_scal, s2));
       pend(9, s2);
     }
     pbeg(1, sm);
@@ -1664,6 +1666,20 @@ int ccp_context_create(const ccp_model *m, int nm, double box0, int device, int 
       delete c;
       return CCP_ERR_BAD_INPUT;
     }
+    std::vector<int2> spec;
+    for (int a : vs)
+      for (int b : vs) {
+        const int k = row[a * ns + b];
+        if (k < 0) continue;
+        const double *p = m->vdw[k].p;
+        if (qq[a * ns + b] != 0.0 || p[5] != 0.0 || p[6] != 0.0 || p[7] != 0.0) spec.push_back({a, b});
+      }
+    c->vdw_nspec = (int)spec.size();
+    if (!spec.empty() &&
+        (dalloc(&c->d_vdw_spec, spec.size()) != cudaSuccess ||
+         cudaMemcpy(c->d_vdw_spec, spec.data(), spec.size() * sizeof(int2), cudaMemcpyHostToDevice) !=
+             cudaSuccess))
+      return fail("2-body site pairs");
     c->vdw_nrows = (int)m->vdw.size();
     c->vdw_nv = (int)vs.size();
     if (dalloc(&c->d_vdw_row, row.size()) != cudaSuccess || dalloc(&c->d_vdw_site, vs.size()) != cudaSuccess ||

@@ -273,7 +273,8 @@ cudaError_t launch_md_wrap(int nm, double *x, double *y, double *z, double box, 
 cudaError_t launch_vdw(const double *xs, const double *ys, const double *zs, int ld,
                        const int *nbr, const double4 *nbrv, const int *ncnt, int cap, int nm,
                        int ns, double rcutsd, const int *row, const double *qq,
-                       const double *par, int nrows, const int *vsite, int nv, double *f,
+                       const double *par, int nrows, const int *vsite, int nv, const int2 *spec,
+                       int nspec, double *f,
                        double *scal, cudaStream_t st);
 cudaError_t launch_prep(const double *x, const double *y, const double *z, const double *xs,
                         const double *ys, const double *zs, int nm, int ld, SiteSets S,
