@@ -333,6 +333,7 @@ bool ensure_fs3_pairs(ccp_context *c, int pair_cap, int vcap) {
   B = Fs3PairBufs{};
   c->fpair_near = 0;
   const size_t np = pair_cap;
+  if (np * 4 * kFs3PairTab > 0xffffffffu) return false;  // a visit's table offsets are 32-bit
   size_t size = 0;
   auto place = [&](size_t bytes) {  // offset of the next buffer, on a 256-byte boundary
     const size_t at = size;

@@ -20,13 +20,22 @@
 // Work of a visit (sites 1..16 of a molecule are numbered 0..15 in the code, in the types
 // [0,1] [2,3] [4..7] [8..11] [12..15]; site 0 is a type of its own): a block's four warps take
 // an 8 x 8 tile of the 16 x 16 site pairs each, as mma.m8n8k4 per type of c and power pair.
-// The types of four sites fill the instruction's K; those of two and one are padded with
-// zeros, which costs 24 instructions per tile where 17 would do, and keeps every lane on the
-// same short loop.  The 33 pairs with a site 0 come from the operand fragments that the warps
+// The types of four sites fill the instruction's K; the two of two sites share a fragment and
+// are padded with zeros (20 instructions per tile where 16 would do, without a branch); the one
+// site of type 0 is multiplied out.  The 33 pairs with a site 0 come from the operand fragments that the warps
 // hold anyway, as products with the other molecule's row of site 0 (one of the four 8-site
 // edges per warp).  No warp waits for another: each adds its own tile's forces.
 // DFMA and DMMA share one pipe on this part (36.8 TFLOP/s DMMA, 34 DFMA); DMMA is taken for
 // its operand reuse: two 16-byte loads per lane feed 32 DFMA's worth.
+//
+// FS3 with its lists at 512 / 2048 waters: 1220 / 6928 us by triples, 750 / 4190 here (at 512:
+// lists and tables 67, pair kernel 483, energies 204; four blocks of four warps per SM, 128
+// registers a thread).  The pair kernel keeps the FP64 pipe 42 % busy: it waits for its
+// own short dependent chains and loads that hit L1 (half of its sectors; the other warps'
+// prefetch brings them).  Measured and worse: table stages by TMA or by the block with barriers
+// (0.54 to 1.7 ms), 3 or 5 blocks per SM, prefetching two visits ahead (547) or the next pass's
+// first visit (494).  The energy kernel keeps it 55 % busy; runs of triples per block, for their
+// shared tables' sake, took 218.
 #include "ccp_device.cuh"
 
 // Pair blocks per SM that the register allocation targets.
