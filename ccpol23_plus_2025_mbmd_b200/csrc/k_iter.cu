@@ -8,7 +8,7 @@
 // order of the reference's recurrence, ewald.f90:960-1010): a (site, k-vector) phase is then
 // one complex product of two table entries, and the tables (nlm + nz per site) stay in L2
 // where the full (site, k) matrix would not.  Each iteration then is
-//   A  blocks [0, nA):  T.mu, one warp per polarisable site, lanes over its (neighbour, site)
+//   A  blocks [0, nA):  T.mu, two warps per polarisable site, lanes over its (neighbour, site)
 //                       tensor entries (contiguous, so the loads coalesce); these blocks also
 //                       clear the S(k) buffer of the other step parity;
 //      blocks [nA, ..): dipole structure factors -4 a(k) S(k), S(k) = sum_s (k.mu_s)
@@ -22,7 +22,8 @@
 //      of a graph body that unrolls several steps then returns at once) and, inside the
 //      graph, sets the WHILE node's condition.  S(k) alternates between two buffers by step
 //      parity, so no block has to clear it after the gather.
-// Small boxes run the whole solve in one cluster instead (k_dip_cluster).  The step normally
+// Small boxes run the whole solve in one cluster instead (k_dip_cluster), middle ones in one
+// cooperative grid (k_dip_grid).  The step normally
 // runs in the row form (k_iter_a_rows, k_iter_b_rows below), which takes the
 // reciprocal sums as matrix products over the rows of the k-vector list.  k_iter_a and k_iter_b
 // take them k-vector by k-vector, from the factor tables (k_max above the row form's) or, by
@@ -1272,6 +1273,11 @@ __global__ void __launch_bounds__(kCluThreads) k_dip_cluster(IterArgs A) {
 // combinations that the gather takes, AD[row][n][(re), (im)] = (S(n) + S(-n), S(n) - S(-n)).
 // Data of other blocks is read past L1 (__ldcg).  A barrier's wait is bounded: a block that
 // waits longer marks the solve as failed and leaves, and the host takes the step kernels.
+// Loop, alone / in the evaluation: 128 waters (29 steps) 327 / 421 us as step kernels, 247 / 329
+// here; 512 (28 steps) 562 / 1220, 424 / 506; 512, PCG 293 / 972, 205 / 255.  Of a step's 15 us
+// at 512 waters the vector and T.mu take 6.8, the gather 3.7 and the two barriers 3.8 (release
+// and acquire through L2; polls without acquire took longer).  The form ends where the vector
+// and the operands no longer fit in shared memory.
 constexpr int kGridThreads = 256, kGridWarps = kGridThreads / 32, kGridRowWarps = 4;
 constexpr int kGridSub = 16;     // sites that a row warp stages at a time
 constexpr int kGridStages = 4;  // stages of its ring, where a step's operands do not all stay

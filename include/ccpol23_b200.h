@@ -41,7 +41,8 @@ extern "C" {
 /* precision forms of a context */
 #define CCP_FP64 0   /* plain FP64 everywhere */
 #define CCP_MIXED 1  /* FP32 for FS2's spectator terms (and, with option
-                        "fs3_fp32_passes", for two of the three FS3 gradient passes); the
+                        "fs3_fp32_passes", for two of the three FS3 gradient passes where FS3
+                        runs by triples); the
                         induced dipoles by preconditioned conjugate gradients in FP64 to
                         1e-8 D RMS (option "dipole_solver"); FP64 for FS3, Ewald, the
                         induction fields and forces, and all sums */
@@ -387,10 +388,16 @@ int ccp_context_phase_ms(const ccp_context *ctx, double *ms, int n);
 
 /* Execution options of the induced-dipole solve (results do not depend on them beyond
    round-off):
-     "graph_loop"    1 (default): the Jacobi loop runs as one CUDA graph with a conditional
-                     WHILE node, no host round trip per iteration; 0: the host launches each
-                     iteration and reads the convergence state (profilers that cannot see
-                     kernels inside conditional graphs need this);
+     "graph_loop"    1 (default): the solve runs without host round trips: as one
+                     thread-block cluster (Jacobi in small boxes, some 45 waters; query
+                     "dipole_cluster_active"), as one cooperative grid (up to some 1000 waters;
+                     option "dipole_grid"), or as a CUDA graph with a conditional WHILE node
+                     over the step kernels; 0: the host launches each iteration and reads the
+                     convergence state (profilers that cannot see kernels inside conditional
+                     graphs need this);
+     "dipole_grid"   1 (default): the cooperative grid is used where it applies and no other
+                     such solve is under way on the device; 0: never.  Query
+                     "dipole_grid_active" tells whether the last solve used it;
      "overlap"       1 (default): FS2 and FS3 run on low-priority side streams concurrently
                      with the Ewald and induction kernels (on a high-priority stream);
      "fs3_triples_per_block"  8 (default): FS3 triples per block when overlapping, so that
@@ -399,33 +406,35 @@ int ccp_context_phase_ms(const ccp_context *ctx, double *ms, int n);
                      blocks per SM (a persistent grid on that many slots), leaving the rest
                      of each SM to the Ewald and induction kernels;
      "fs3_param_grad" 0 (default): see ccp_context_fs3_param_grad;
+     "fs3_pair_form" 1 (default): in boxes wider than two FS3 cut-offs (12.6 A) FS3 runs by
+                     molecule pairs (FP64); 0: by triples, as in smaller boxes.  Query
+                     "fs3_pair_form_active" tells which ran;
      "phase_matrix"  1 (default): the polarisable sites' phases are tabulated once per
                      evaluation as exp(i(l x + m y)) and exp(i n z) factors (when they take at
                      most 1 GiB), so a (site, k) phase is one complex product; 0: never (the
                      tiled on-the-fly reciprocal kernels run every iteration);
-     "phase_matrix_full" 1 (default): with the factor tables, the full (site, k-vector)
-                     phase matrix is formed once per evaluation when it fits in half of the L2
-                     (38 MB at 512 waters), and the dipole steps read one phase per pair;
-                     0: never.  Query "phase_matrix_full_active" tells whether it was used;
-     "dipole_row_form" 1 (default): without the full phase matrix, the dipole steps take the
-                     reciprocal sums row by row of the k-vector list (one (l, m), a run of n),
-                     so each loaded factor serves many products; 0: one phase per (site,
-                     k-vector) product from the factor tables.  The same sums to rounding.
-                     Query "dipole_row_form_active" tells whether it was used;
+     "phase_matrix_full" 0 (default): never; 1: with the factor tables, the full (site,
+                     k-vector) phase matrix is formed once per evaluation when it fits in half
+                     of the L2 (38 MB at 512 waters), and the dipole steps read one phase per
+                     pair.  Query "phase_matrix_full_active" tells whether it was used;
+     "dipole_row_form" 1 (default): the Ewald sums and, without the full phase matrix, the
+                     dipole steps take the reciprocal sums by rows of the k-vector list (one
+                     (l, m), a run of n) as matrix products (k_max up to 19); 0: one phase per
+                     (site, k-vector).  The same sums to rounding.  Query
+                     "dipole_row_form_active" tells whether the dipole steps used it;
      "dipole_sum_sites" 1..128 (default 32): polarisable sites per structure-factor block of
-                     a dipole step (a tuning option; results unchanged);
+                     a dipole step that is not in the row form (results unchanged);
      "dipole_gather_sites" 2, 3, 4 (default), 6 or 8: polarisable sites per reciprocal-field
-                     block of a dipole step (a tuning option; results unchanged);
+                     block of such a step (results unchanged);
      "dipole_solver" 0 (CCP_FP64 default): the reference's Jacobi iteration and criterion
                      (sum |dmu|^2 < 1e-20 e^2 A^2); 1: preconditioned conjugate gradients
                      (preconditioner diag(alpha), so the convergence quantity is the Jacobi
                      update at the iterate) to the same criterion; 2 (CCP_MIXED default): PCG
                      to an RMS update of 1e-8 D per polarisable site.  PCG needs the phase
                      table; without it the solve is Jacobi.  ind_iters then counts PCG steps;
-     "fs3_fp32_passes" 0 (default): FS3 in FP64 in both forms; 1: in the CCP_MIXED form FS3's
-                     ik and jk gradient passes run in FP32 (about 3 % faster FS3; site forces
-                     within 2e-6 of FP64, but per-molecule forces 1.45e-5 off at 2048
-                     waters, above the mixed form's 1e-5 bar);
+     "fs3_fp32_passes" 0 (default): FS3 in FP64 in both forms; 1: where FS3 runs by triples,
+                     its ik and jk gradient passes run in FP32 in the CCP_MIXED form (site
+                     forces within 2e-6 of FP64); FS3 by pairs is FP64 and faster;
      "fs3_high_priority" 0 (default): FS3's side stream at the low priority (1: at the
                      Ewald/induction chain's high priority);
      "pdl"           1 (default): the two kernels of a dipole step are launched with
