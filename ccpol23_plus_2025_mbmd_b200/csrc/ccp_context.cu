@@ -998,51 +998,64 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
       CK(cudaStreamWaitEvent(sm, c->ev_fork, 0));
       if (kfork) CK(cudaStreamWaitEvent(sk, c->ev_fork, 0));
     }
-    // three-body terms first, so that on side streams they start at once
     double *f3 = side ? c->d_f + (size_t)3 * nm * ns : c->d_f;
     double *gfs3 = nullptr;
     if ((mask & T_FS3) && c->opt_pgrad) {
       gfs3 = c->d_gfs3;
       CK(cudaMemsetAsync(gfs3, 0, sizeof(double) * kFs3GradLen, s3));
     }
-    if (fs3_pair) {
-      pbeg(7, s3);
-      c->launches++;  // two kernels; LK counts one
-      LK(launch_fs3_pair_lists(c->fpair, c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_s17,
-                               c->d_bgr, c->d_tri, c->tri_cap, c->d_icnt, c->nsm, s3));
-      pend(7, s3);
-      pbeg(8, s3);
-      c->launches++;  // two kernels
-      LK(launch_fs3_pair(c->fpair, c->d_icnt, c->d_comb, c->d_s17, c->d_coef, c->d_bgr, F3, nm, ns,
-                         f3, c->d_fc3, c->d_scal, c->d_tri, c->tri_cap, c->nsm, gfs3, s3));
-      pend(8, s3);
-    } else if (mask & T_FS3) {
-      pbeg(7, s3);
-      LK(launch_fs3_enum(c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_tri, c->tri_cap,
-                         c->d_icnt, s3));
-      pend(7, s3);
-      pbeg(8, s3);
-      const int fs3_prec = c->precision == CCP_MIXED && c->opt_fs3_low ? CCP_MIXED : CCP_FP64;
-      LK(launch_fs3(fs3_prec, c->d_tri, c->d_icnt, c->tri_cap, c->d_s17, c->d_coef, c->d_bgr,
-                    nm, ns, f3, c->d_fc3, c->d_scal, c->nsm, side ? c->opt_fs3_tpb : 0,
-                    side ? c->opt_fs3_bps : 0, gfs3,
-                    s3));
-      pend(8, s3);
-    }
-    if (mask & T_FS2) {
-      pbeg(6, s2);
-      LK(launch_fs2_enum(c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F2, c->d_pairs, c->pair_cap,
-                         c->d_icnt, s2));
-      LK(launch_fs2(c->precision, c->d_pairs, c->d_icnt, c->pair_cap, c->d_comb, c->d_s17, c->d_nbr,
-                    c->d_ncnt, c->cap, F2, nm, ns, f3, c->d_fc2, c->d_scal, s2));
-      pend(6, s2);
-    }
-    if (mask & T_VDW) {
-      pbeg(9, s2);
-      LK(launch_vdw(pxs, pys, pzs, ld, c->d_nbr, c->d_nbrv, c->d_ncnt, c->cap, nm, ns,
-                    c->rcutsd, c->d_vdw_row, c->d_vdw_qq, c->d_vdw_par, c->vdw_nrows,
-                    c->d_vdw_site, c->vdw_nv, c->d_vdw_spec, c->vdw_nspec, f3, c->d_scal, s2));
-      pend(9, s2);
+    auto side_terms = [&]() -> int {
+      if (fs3_pair) {
+        pbeg(7, s3);
+        c->launches++;  // two kernels; LK counts one
+        LK(launch_fs3_pair_lists(c->fpair, c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_s17,
+                                 c->d_bgr, c->d_tri, c->tri_cap, c->d_icnt, c->nsm, s3));
+        pend(7, s3);
+        pbeg(8, s3);
+        c->launches++;  // two kernels
+        LK(launch_fs3_pair(c->fpair, c->d_icnt, c->d_comb, c->d_s17, c->d_coef, c->d_bgr, F3, nm, ns,
+                           f3, c->d_fc3, c->d_scal, c->d_tri, c->tri_cap, c->nsm, gfs3, s3));
+        pend(8, s3);
+      } else if (mask & T_FS3) {
+        pbeg(7, s3);
+        LK(launch_fs3_enum(c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F3, c->d_tri, c->tri_cap,
+                           c->d_icnt, s3));
+        pend(7, s3);
+        pbeg(8, s3);
+        const int fs3_prec = c->precision == CCP_MIXED && c->opt_fs3_low ? CCP_MIXED : CCP_FP64;
+        LK(launch_fs3(fs3_prec, c->d_tri, c->d_icnt, c->tri_cap, c->d_s17, c->d_coef, c->d_bgr,
+                      nm, ns, f3, c->d_fc3, c->d_scal, c->nsm, side ? c->opt_fs3_tpb : 0,
+                      side ? c->opt_fs3_bps : 0, gfs3,
+                      s3));
+        pend(8, s3);
+      }
+      if (mask & T_FS2) {
+        pbeg(6, s2);
+        LK(launch_fs2_enum(c->d_comb, c->d_nbr, c->d_ncnt, c->cap, nm, F2, c->d_pairs, c->pair_cap,
+                           c->d_icnt, s2));
+        LK(launch_fs2(c->precision, c->d_pairs, c->d_icnt, c->pair_cap, c->d_comb, c->d_s17, c->d_nbr,
+                      c->d_ncnt, c->cap, F2, nm, ns, f3, c->d_fc2, c->d_scal, s2));
+        pend(6, s2);
+      }
+      if (mask & T_VDW) {
+        pbeg(9, s2);
+        LK(launch_vdw(pxs, pys, pzs, ld, c->d_nbr, c->d_nbrv, c->d_ncnt, c->cap, nm, ns,
+                      c->rcutsd, c->d_vdw_row, c->d_vdw_qq, c->d_vdw_par, c->vdw_nrows,
+                      c->d_vdw_site, c->vdw_nv, c->d_vdw_spec, c->vdw_nspec, f3, c->d_scal, s2));
+        pend(9, s2);
+      }
+      return CCP_OK;
+    };
+    // The side terms are launched after the chain's kernels up to the dipole solve, so that the
+    // chain, the longer path in small boxes, neither waits for their launches nor for SM slots
+    // behind their blocks: 37 waters from host arrays 433 -> 347 us, 128 553 -> 484, 1003 (mixed)
+    // 2390 -> 2350; 512 and 2048 are the same either way.  FS3's gradient form, whose blocks stay
+    // for the whole kernel and are the longer path, goes first (256 waters with its backward pass
+    // 2360 against 2660 us).
+    const bool side_late = side && (mask & T_INDUCTION) && !gfs3;
+    if (!side_late) {
+      const int r = side_terms();
+      if (r) return r;
     }
     pbeg(1, sm);
     if (mask & (T_RSPACE | T_INDUCTION)) {
@@ -1129,6 +1142,10 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
                              sm));
       pend(3, sm);
       pbeg(4, sm);
+      if (side_late) {
+        const int r = side_terms();
+        if (r) return r;
+      }
       {
         int r = run_dipole_loop(c, sm);
         if (r) return r;
