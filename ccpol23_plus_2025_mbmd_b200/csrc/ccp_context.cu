@@ -757,20 +757,21 @@ int try_dip_grid(ccp_context *c, const IterArgs &A, cudaStream_t st, bool *done)
 
 // The whole Jacobi solve from mu = 0.  The state {iterations, change, energy} is copied to
 // h_istate; in the graph form the copy completes at the evaluation's final synchronisation.
-int run_dipole_loop(ccp_context *c, cudaStream_t st) {
+// steps_only: not as one cluster or grid.
+int run_dipole_loop(ccp_context *c, cudaStream_t st, bool steps_only) {
   // the first step writes every dipole, so d_mu needs no clearing
   const bool pcg = pcg_solver(c);
   c->pcg_active = pcg;
   if (pcg && !c->d_pcg) CK(dalloc(&c->d_pcg, 4 * (size_t)c->nm * c->S.np * 3));
   c->grid_active = false;
   const IterArgs A1 = make_iter_args(c, 0, 0, 0);
-  if (c->opt_graph && dip_cluster(c, A1)) {
+  if (c->opt_graph && !steps_only && dip_cluster(c, A1)) {
     if (!cuda_ok(launch_dip_cluster(A1, st), "dipole solve")) return CCP_ERR_CUDA;
     CK(cudaMemcpyAsync(c->h_istate, c->d_istate, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     c->ind_per_iter = 0;
     return CCP_OK;
   }
-  if (c->opt_graph) {
+  if (c->opt_graph && !steps_only) {
     bool done = false;
     CK(cudaMemsetAsync(c->d_istate, 0, kIterStateLen * sizeof(double), st));
     const int r = try_dip_grid(c, A1, st, &done);
@@ -1147,7 +1148,10 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
         if (r) return r;
       }
       {
-        int r = run_dipole_loop(c, sm);
+        // FS3's gradient form by triples fills every SM's shared memory until it ends: the one-
+        // kernel solves would wait for it, the step kernels' blocks fit beside it (48 waters
+        // with the backward pass: 2153 us against 2039 before those forms)
+        int r = run_dipole_loop(c, sm, side && gfs3 && !fs3_pair);
         if (r) return r;
       }
       pend(4, sm);
