@@ -273,12 +273,17 @@ __device__ __forceinline__ void fs3_visits(int i, const double4 *__restrict__ co
     const int branch = ravg <= P.rmin ? 0 : (ravg >= P.rmax ? 1 : 2);
     if (branch == 2) atomicAdd(&icnt[C_NBLEND_FS3], 1);
     const int slot = atomicAdd(&icnt[C_NTRI_FS3], 1);
+    if (slot >= tri_cap) continue;  // the host grows the list and re-runs
     const int pij = lr[a], pik = lr[c], pjk = pair_of(near, head[j], cap, j, k);
-    if (pjk < 0) {  // no such pair within the widened radius: the host takes the triple form
-      atomicAdd(&icnt[C_FS3_MISS], 1);
+    if (pjk < 0 || max(max(pij, pik), pjk) >= pair_cap) {
+      // no such pair within the widened radius (the host takes the triple form), or no room for
+      // one of the pairs (it grows the list): the evaluation is repeated.  Every counted record
+      // is written all the same, this one with the valid indices 0 and no weight: a reader of
+      // the list must not meet what the memory held before.
+      if (pjk < 0) atomicAdd(&icnt[C_FS3_MISS], 1);
+      tri[slot] = Triple{};
       continue;
     }
-    if (max(max(pij, pik), pjk) >= pair_cap || slot >= tri_cap) continue;  // the host grows the lists and re-runs
     // global damping and switch (threebody_potential.f90:898-904, 1418-1423)
     const double pom = exp(P.alp3 * (ravg - P.r0dmp));
     const double ppom = 1.0 / (1.0 + pom);
@@ -333,6 +338,13 @@ __global__ void __launch_bounds__(128)
     fs3_visits(blockIdx.x, comb, near, head, cap, P, vis, vcnt, vcap, pair_cap, tri, tri_cap, icnt);
   else
     fs3_tables(blockIdx.x - nm, gridDim.x - nm, pairv, pairij, icnt, pair_cap, s17, bgr, tab, wtab);
+}
+
+// Whether the lists hold every pair, visit and triple that was found.  If not, the host repeats
+// the evaluation and the kernels that use the lists have nothing to do.
+__device__ __forceinline__ bool fs3_lists_whole(const int *__restrict__ icnt, int pair_cap) {
+  return icnt[C_NPAIR_FS3] <= pair_cap && icnt[C_FS3_VMAX] == 0 && icnt[C_FS3_MISS] == 0 &&
+         icnt[C_OVERFLOW] == 0;
 }
 
 // D = A (8x4) B (4x8) + C in FP64: lane l holds A[l/4][l%4], B[l%4][l/4] and C, D
@@ -682,6 +694,7 @@ __global__ void __launch_bounds__(kPT, GRAD ? 2 : CCP_FS3_PAIR_BLOCKS)
   PairGrad *GS = reinterpret_cast<PairGrad *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int np = min(icnt[C_NPAIR_FS3], pair_cap);
+  if (!fs3_lists_whole(icnt, pair_cap)) return;
   if (GRAD) {
     for (int t = tid; t < 2 * kCoef; t += kPT) (&GS->gc[0][0])[t] = 0.0;
     for (int t = tid; t < 2 * 3 * kTab; t += kPT) (&GS->gb[0][0][0])[t] = 0.0;
@@ -833,6 +846,7 @@ __global__ void __launch_bounds__(kET, CCP_FS3_ENERGY_BLOCKS)
                  const double *__restrict__ vpart, int pair_cap, Fs3Params P, int nm, double *fc3,
                  double *scal, int *icnt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (!fs3_lists_whole(icnt, pair_cap)) return;
   double *Cs = reinterpret_cast<double *>(smem_raw);  // [2][216][kCs]
   for (int t = threadIdx.x; t < 2 * kCoef / 2; t += kET) {
     const double2 c = __ldg(reinterpret_cast<const double2 *>(coef) + t);
