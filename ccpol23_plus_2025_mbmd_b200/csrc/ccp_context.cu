@@ -1216,8 +1216,7 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
     if (ic[C_OVERFLOW] > 0) {
       ncap = std::min(nm, ic[C_OVERFLOW] + 32);
       grow = true;
-    }
-    if (fs3_pair) {
+    } else if (fs3_pair) {  // of a short neighbour list the pairs say nothing
       const int npair = ic[C_NPAIR_FS3], vmax = ic[C_FS3_VMAX];
       if (ic[C_FS3_MISS] > 0) {
         fs3_pair = false;

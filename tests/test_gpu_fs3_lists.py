@@ -42,6 +42,28 @@ def _triples(m, b):
         return _fs3(c, b)
 
 
+def _with_rcut(tmp_path, rcut):
+    """The FS3 model with another cut-off radius in its CONTROL."""
+    for p in data_dir("fs3").iterdir():
+        t = p.read_text()
+        if p.name == "CONTROL":
+            assert t.count("9.0                 # rcut ") == 1
+            t = t.replace("9.0                 # rcut ", f"{rcut:.1f}                # rcut ")
+        (tmp_path / p.name).write_text(t)
+    return Model(tmp_path)
+
+
+def test_neighbour_list_overflow(product, tmp_path):
+    """A neighbour list that outgrows its first 192 entries per molecule lacks pairs of triples
+    that it holds; the evaluation that follows with a longer list still goes by pairs."""
+    m = _with_rcut(tmp_path, 12.0)
+    b = water_box(m, 300, 20.79, 702, ld=28)  # 244 neighbours per molecule
+    ref = _triples(m, b)
+    with Context(m, b.nm, b.box) as c:
+        _compare(_fs3(c, b), ref)
+        assert c.get_option("fs3_pair_form_active") == 1
+
+
 @pytest.mark.parametrize("grad", [0, 1])
 @pytest.mark.parametrize("before", [None, 0, 1])
 def test_pair_list_overflow(product, before, grad):
