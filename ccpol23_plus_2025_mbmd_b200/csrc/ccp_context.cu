@@ -569,7 +569,7 @@ IterArgs make_iter_args(ccp_context *c, cudaGraphConditionalHandle handle, int u
     A.XY = nullptr;
     A.rows = c->d_rows;
     A.nrow = c->nrow;
-    A.row_sites = iter_row_sites(A.nw, c->nrow);
+    A.row_sites = iter_row_sites(A.nw, c->nrow, c->kmax[2]);
     A.zs = 8 * iter_row_tiles(c->kmax[2]);
     A.XYr = c->d_P;
     A.Zc = reinterpret_cast<const double *>(c->d_P + (size_t)((c->nrow + 7) / 8 * 8) * A.nw);

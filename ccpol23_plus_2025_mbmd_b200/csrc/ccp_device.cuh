@@ -322,7 +322,7 @@ cudaError_t launch_tmu(const int *nbr, const int *ncnt, int cap, int nm, int np,
                        double *eim, cudaStream_t st);
 int iter_row_tiles(int nmax);
 bool iter_rows_fit(int nmax);
-int iter_row_sites(int nw, int nrow);
+int iter_row_sites(int nw, int nrow, int nmax);
 // zs = 8 iter_row_tiles(kn) doubles per site in Zc.
 cudaError_t launch_phase_rows(const double2 *tab, int nm, SiteSets S, int kl, int km, int kn,
                               const KRow *rows, int nrow, int zs, double2 *XYt, double *Zc,

@@ -2032,25 +2032,35 @@ cudaError_t launch_step(Kernel kernel, int blocks, const IterArgs &A, cudaStream
 int iter_row_tiles(int nmax) { return nmax / 4 + 1; }
 bool iter_rows_fit(int nmax) { return iter_row_tiles(nmax) <= kRowTilesMax; }
 
-// Sites of a structure-factor block: 96 (six steps per warp, their XY loaded ahead) while that
-// makes no more than a few waves of blocks, so that the atomics stay few; 48 in small boxes,
-// where blocks are too few otherwise.
-int iter_row_sites(int nw, int nrow) {
-  const int nt8 = (nrow + 7) / 8;
-  int cs = nw <= 512 ? 48 : 96;
-  while ((long long)nt8 * ((nw + cs - 1) / cs) > 148 * 8) cs *= 2;
-  return cs;
-}
-
 // Up to this many sites per block, their Zc fit the shared memory that the warps' sums take
 // at the end; longer blocks read them from memory, where they overlap with the products.
 constexpr int kRowStage = 96;
+// Shared memory of k_iter_a_rows with `tiles` n tiles: the dipoles, and the sums or the staged Zc.
+constexpr size_t iter_rows_smem(int sites, int tiles) {
+  const size_t sums = sizeof(double2) * kWarps * 4 * tiles * 32,
+               zc = sites <= kRowStage ? sizeof(double) * sites * (8 * tiles + 2) : 0;
+  return sizeof(double4) * sites + (sums > zc ? sums : zc);
+}
+constexpr size_t kRowSmemMax = 226 * 1024;  // 1 KB for the static arrays
+static_assert(iter_rows_smem(kRowStage, kRowTilesMax) <= kRowSmemMax, "the smallest blocks fit");
+
+// Sites of a structure-factor block: 96 (six steps per warp, their XY loaded ahead) while that
+// makes no more than a few waves of blocks, so that the atomics stay few; 48 in small boxes,
+// where blocks are too few otherwise.  Larger boxes take as many as fit in shared memory (3072
+// with five n tiles) and more waves.
+int iter_row_sites(int nw, int nrow, int nmax) {
+  const int nt8 = (nrow + 7) / 8, tiles = iter_row_tiles(nmax);
+  int cs = nw <= 512 ? 48 : 96;
+  while ((long long)nt8 * ((nw + cs - 1) / cs) > 148 * 8 &&
+         iter_rows_smem(2 * cs, tiles) <= kRowSmemMax)
+    cs *= 2;
+  return cs;
+}
+
 template <int J>
 cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
   const bool zs = A.row_sites <= kRowStage;
-  const size_t smem = sizeof(double4) * A.row_sites +
-                      std::max(sizeof(double2) * kWarps * 4 * J * 32,
-                               zs ? sizeof(double) * (size_t)A.row_sites * (8 * J + 2) : 0);
+  const size_t smem = iter_rows_smem(A.row_sites, J);
   const auto k = zs ? (A.cu ? k_iter_a_rows<true, J, true> : k_iter_a_rows<false, J, true>)
                     : (A.cu ? k_iter_a_rows<true, J, false> : k_iter_a_rows<false, J, false>);
   if (smem > 48 * 1024) {
