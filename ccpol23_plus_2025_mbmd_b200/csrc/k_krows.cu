@@ -373,6 +373,7 @@ cudaError_t set_smem(F kern, size_t smem) {
 template <bool DIP, int J>
 cudaError_t sums_t(const KRowArgs &A, const double *mu, cudaStream_t st) {
   const int k1 = k1_of(A.kl, A.km, A.kn), total = A.nm * (DIP ? A.S.np : A.S.nq);
+  if (total <= 0) return cudaErrorInvalidConfiguration;  // no such site: a grid of no blocks
   const int ny = ((A.nrow + 7) / 8 + kWarps - 1) / kWarps, chunks = (total + kCh - 1) / kCh;
   // blocks for two per SM; each keeps its row tiles' sums over all chunks of its split
   int nx = (148 * 2 + ny - 1) / ny;
