@@ -197,7 +197,9 @@ struct ccp_context {
   double2 *d_PM = nullptr;
   size_t PM_cap = 0;
   bool use_PM = false;
-  int opt_pm = 0;  // the full phase matrix when it fits (1) or never (0)
+  // the full phase matrix when it fits (1), where the row form does not run besides (2), or
+  // never (0)
+  int opt_pm = 2;
   // without the full phase matrix, the row form of the dipole step (1) or the factor-table
   // kernels (0)
   int opt_rows = 1;
@@ -520,8 +522,7 @@ struct EvalOut {
 // polarisable site: 5 MB at 512 waters, 46 MB at 2048).
 constexpr size_t kPhaseBudget = size_t(1) << 30;
 // The full phase matrix (16 bytes per polarisable site and k-vector: 38 MB at 512 waters,
-// 568 MB at 2048), an option, is used when it fits in half of the L2, which it is read from
-// twice per step.
+// 568 MB at 2048) is used when it fits in half of the L2, which it is read from twice per step.
 size_t full_phase_budget(const ccp_context *c) { return c->l2_bytes / 2; }
 
 constexpr double kIndThr = 1.0e-20;  // iteridm convergence threshold on sum |dmu|^2
@@ -827,8 +828,13 @@ int ensure_phase_matrix(ccp_context *c) {
   c->use_P = c->opt_phase && c->nk > 0 && n * sizeof(double2) <= kPhaseBudget &&
              2 * c->kmax[2] + 1 <= 255;
   const size_t npm = (size_t)c->nm * c->S.np * (size_t)c->nk;
-  c->use_PM = c->use_P && c->opt_pm && npm * sizeof(double2) <= full_phase_budget(c);
-  c->use_rows = c->use_P && !c->use_PM && c->opt_rows && iter_rows_fit(c->kmax[2]);
+  // The row form is the fastest where it applies; past its k_max, or without it, the matrix
+  // where it fits: 37 waters at k_max 20 take 2263 us with it and 3177 on the factor tables, 64
+  // waters 2524 and 3580.
+  const bool rows = c->use_P && c->opt_rows && iter_rows_fit(c->kmax[2]);
+  c->use_PM = c->use_P && (c->opt_pm == 1 || (c->opt_pm == 2 && !rows)) &&
+              npm * sizeof(double2) <= full_phase_budget(c);
+  c->use_rows = rows && !c->use_PM;
   if (c->use_P && n > c->P_cap) {
     if (c->d_P) cudaFree(c->d_P);
     c->d_P = nullptr;
@@ -1797,7 +1803,7 @@ int ccp_context_set_option(ccp_context *ctx, const char *name, int value) {
   } else if (n == "phase_matrix") {
     ctx->opt_phase = value != 0;
   } else if (n == "phase_matrix_full") {
-    ctx->opt_pm = value != 0;
+    ctx->opt_pm = value == 2 ? 2 : value != 0;
   } else if (n == "dipole_row_form") {
     ctx->opt_rows = value != 0;
   } else if (n == "dipole_sum_sites") {

@@ -413,10 +413,11 @@ int ccp_context_phase_ms(const ccp_context *ctx, double *ms, int n);
                      evaluation as exp(i(l x + m y)) and exp(i n z) factors (when they take at
                      most 1 GiB), so a (site, k) phase is one complex product; 0: never (the
                      tiled on-the-fly reciprocal kernels run every iteration);
-     "phase_matrix_full" 0 (default): never; 1: with the factor tables, the full (site,
-                     k-vector) phase matrix is formed once per evaluation when it fits in half
-                     of the L2 (38 MB at 512 waters), and the dipole steps read one phase per
-                     pair.  Query "phase_matrix_full_active" tells whether it was used;
+     "phase_matrix_full" 1: with the factor tables, the full (site, k-vector) phase matrix is
+                     formed once per evaluation when it fits in half of the L2 (38 MB at 512
+                     waters), and the dipole steps read one phase per pair; 2 (default): so
+                     where the row form below does not run; 0: never.  Query
+                     "phase_matrix_full_active" tells whether it was used;
      "dipole_row_form" 1 (default): the Ewald sums and, without the full phase matrix, the
                      dipole steps take the reciprocal sums by rows of the k-vector list (one
                      (l, m), a run of n) as matrix products (k_max up to 19); 0: one phase per
