@@ -829,8 +829,8 @@ int ensure_phase_matrix(ccp_context *c) {
              2 * c->kmax[2] + 1 <= 255;
   const size_t npm = (size_t)c->nm * c->S.np * (size_t)c->nk;
   // The row form is the fastest where it applies; past its k_max, or without it, the matrix
-  // where it fits: 37 waters at k_max 20 take 2263 us with it and 3177 on the factor tables, 64
-  // waters 2524 and 3580.
+  // where it fits: 37 waters at k_max 20 take 2272 us with it and 3177 on the factor tables, 64
+  // waters 2500 and 3580.
   const bool rows = c->use_P && c->opt_rows && iter_rows_fit(c->kmax[2]);
   c->use_PM = c->use_P && (c->opt_pm == 1 || (c->opt_pm == 2 && !rows)) &&
               npm * sizeof(double2) <= full_phase_budget(c);

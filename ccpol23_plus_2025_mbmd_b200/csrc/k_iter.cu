@@ -378,19 +378,34 @@ __device__ __forceinline__ void iter_a_tmu(const IterArgs &A, int block, int nA)
   }
 }
 
+// Without rows T.mu takes one warp per polarisable site: iter_a_tmu's entries held ahead cost the
+// sums' blocks of the same kernel their occupancy (96 registers a thread against 56, PCG 128
+// against 72), and those are most of this step.
 template <bool PCG, bool PM>
 __global__ void __launch_bounds__(kThreads)
     k_iter_a(IterArgs A) {
   // no test of the finished flag here: a step after the finish only rewrites the T.mu
   // scratch and S(k), which the next use clears, and it saves a dependent load per step
-  const int nA = tmu_blocks(A.nw);
-  if ((int)blockIdx.x < nA) {
-    iter_a_tmu<PCG>(A, blockIdx.x, nA);
-    return;
-  }
   pdl_wait();  // the previous step's dipoles (and its gather's last use of the S(k) buffer)
+  const int nA = (A.nw + kWarps - 1) / kWarps;
   PcgIn pin;
   if constexpr (PCG) pin = pcg_in(A);
+  if ((int)blockIdx.x < nA) {
+    // these blocks also clear the S(k) buffer of the other step parity
+    double2 *other = reinterpret_cast<double2 *>(A.sk) + (A.par ^ 1);
+    for (int k = blockIdx.x * kThreads + threadIdx.x; k < A.nk; k += nA * kThreads)
+      other[2 * (size_t)k] = make_double2(0.0, 0.0);
+    const int w = blockIdx.x * kWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (w >= A.nw) return;
+    double ex, ey, ez;
+    if constexpr (PCG)
+      tmu_warp(w, lane, A.nbr, A.ncnt, A.cap, A.np, A.T4, A.TB, A.S4, A.SB, pin, ex, ey, ez);
+    else
+      tmu_warp(w, lane, A.nbr, A.ncnt, A.cap, A.np, A.T4, A.TB, A.S4, A.SB, MuIn{A.mu}, ex, ey, ez);
+    pdl_launch_dependents();  // as late as in iter_a_tmu
+    if (lane < 3) A.eim[(size_t)w * 3 + lane] = lane == 0 ? ex : (lane == 1 ? ey : ez);
+    return;
+  }
   // structure factors: block b covers k-vectors [kt*256, kt*256+256) and sites of chunk sc
   extern __shared__ double smu[];  // A.sum_sites x 3 dipole components
   const int b = blockIdx.x - nA;
@@ -2072,10 +2087,9 @@ cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
 
 cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st) {
   if (A.sum_sites < 1 || A.sum_sites > kSumSitesMax) return cudaErrorInvalidValue;
-  const int nA = tmu_blocks(A.nw);
   const int nsc = (A.nw + A.sum_sites - 1) / A.sum_sites;
   if (A.rows) {
-    const int nb = nA + (A.nrow + 7) / 8 * ((A.nw + A.row_sites - 1) / A.row_sites);
+    const int nb = tmu_blocks(A.nw) + (A.nrow + 7) / 8 * ((A.nw + A.row_sites - 1) / A.row_sites);
     switch (iter_row_tiles(A.nmax)) {
       case 1: return launch_iter_a_rows<1>(A, nb, st);
       case 2: return launch_iter_a_rows<2>(A, nb, st);
@@ -2087,7 +2101,7 @@ cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st) {
   }
   const size_t smem = sizeof(double) * 3 * A.sum_sites;
   const int nkt = (A.nk + kThreads - 1) / kThreads;
-  const int nb = nA + nkt * nsc;
+  const int nb = (A.nw + kWarps - 1) / kWarps + nkt * nsc;
   if (A.PM)
     return A.cu ? launch_step(k_iter_a<true, true>, nb, A, st, smem)
                 : launch_step(k_iter_a<false, true>, nb, A, st, smem);
