@@ -178,6 +178,7 @@ struct ccp_context {
   unsigned *d_ticket = nullptr;  // last-block ticket of the fused update kernel
   std::array<int, 5> clu_key{};  // sizes that clu_fits was asked for
   bool clu_fits = false;         // the solve in one cluster applies to them
+  bool clu_active = false;       // the last solve ran in one cluster
   std::array<int, 6> grid_key{};  // sizes that grid_blocks was asked for
   int grid_blocks = 0;           // blocks of the solve in one grid, 0 where it does not apply
   int opt_grid = 1;              // the solve in one grid (k_dip_grid) where it applies
@@ -764,10 +765,11 @@ int run_dipole_loop(ccp_context *c, cudaStream_t st, bool steps_only) {
   const bool pcg = pcg_solver(c);
   c->pcg_active = pcg;
   if (pcg && !c->d_pcg) CK(dalloc(&c->d_pcg, 4 * (size_t)c->nm * c->S.np * 3));
-  c->grid_active = false;
+  c->clu_active = c->grid_active = false;
   const IterArgs A1 = make_iter_args(c, 0, 0, 0);
   if (c->opt_graph && !steps_only && dip_cluster(c, A1)) {
     if (!cuda_ok(launch_dip_cluster(A1, st), "dipole solve")) return CCP_ERR_CUDA;
+    c->clu_active = true;
     CK(cudaMemcpyAsync(c->h_istate, c->d_istate, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     c->ind_per_iter = 0;
     return CCP_OK;
@@ -1895,7 +1897,7 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
   } else if (n == "dipole_grid_active") {
     *value = ctx->grid_active;
   } else if (n == "dipole_cluster_active") {
-    *value = ctx->opt_graph && ctx->clu_fits;
+    *value = ctx->clu_active;
   } else if (n == "dipole_solver") {
     *value = ctx->opt_solver;
   } else if (n == "cell_list") {
