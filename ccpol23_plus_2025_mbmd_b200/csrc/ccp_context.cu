@@ -182,6 +182,7 @@ struct ccp_context {
   std::array<int, 6> grid_key{};  // sizes that grid_blocks was asked for
   int grid_blocks = 0;           // blocks of the solve in one grid, 0 where it does not apply
   int opt_grid = 1;              // the solve in one grid (k_dip_grid) where it applies
+  int opt_grid_polls = 1 << 21;  // polls of one of its waits before it gives up, about a second
   bool grid_failed = false;      // a wait in it ran out: the step kernels from then on
   bool grid_active = false;      // the last solve ran in one grid
   double *d_grid = nullptr;
@@ -745,7 +746,7 @@ int try_dip_grid(ccp_context *c, const IterArgs &A, cudaStream_t st, bool *done)
     }
     CK(e);
   }
-  const cudaError_t e = launch_dip_grid(A, c->grid_blocks, c->d_grid, st);
+  const cudaError_t e = launch_dip_grid(A, c->grid_blocks, c->opt_grid_polls, c->d_grid, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     (void)cudaGetLastError();
     c->grid_failed = true;
@@ -1800,6 +1801,14 @@ int ccp_context_set_option(ccp_context *ctx, const char *name, int value) {
   const std::string n(name);
   if (n == "dipole_grid") {
     ctx->opt_grid = value != 0;
+    ctx->grid_failed = false;
+  } else if (n == "dipole_grid_polls") {
+    if (value < 1) {
+      set_error("ccp_context_set_option: dipole_grid_polls must be positive");
+      return CCP_ERR_BAD_INPUT;
+    }
+    ctx->opt_grid_polls = value;
+    ctx->grid_failed = false;
   } else if (n == "graph_loop") {
     ctx->opt_graph = value != 0;
   } else if (n == "phase_matrix") {
@@ -1894,6 +1903,8 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
     *value = ctx->use_rows ? 1 : 0;
   } else if (n == "dipole_grid") {
     *value = ctx->opt_grid;
+  } else if (n == "dipole_grid_polls") {
+    *value = ctx->opt_grid_polls;
   } else if (n == "dipole_grid_active") {
     *value = ctx->grid_active;
   } else if (n == "dipole_cluster_active") {

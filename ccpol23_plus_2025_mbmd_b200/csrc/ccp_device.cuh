@@ -342,16 +342,17 @@ cudaError_t launch_dip_cluster(const IterArgs &A, cudaStream_t st);
 // most one per SM (0: the form does not take these sizes; asked once per set of sizes), its
 // scratch in doubles, and its launch.  The blocks wait for one another, so two such kernels must
 // not be under way at the same time on a device (the caller orders them); A.state[kIterFinished]
-// is -1 afterwards if a wait ran out.
+// is -1 afterwards if a wait ran out, which it does after `polls` of the counter.
 struct GridArgs {
   double *ad, *acc;
-  unsigned *bar;
+  unsigned *bar, polls;
   int ns, nchunk, chunk;  // sites per block; chunks of the sites, sites per chunk
   int stages, stay;       // of the operand ring; all of a step's operands stay in it
 };
 int dip_grid_blocks(const IterArgs &A, int nsm);
 size_t dip_grid_scratch(const IterArgs &A);
-cudaError_t launch_dip_grid(const IterArgs &A, int blocks, double *scratch, cudaStream_t st);
+cudaError_t launch_dip_grid(const IterArgs &A, int blocks, unsigned polls, double *scratch,
+                            cudaStream_t st);
 cudaError_t launch_iter_a(const IterArgs &A, cudaStream_t st);
 cudaError_t launch_iter_b(const IterArgs &A, cudaStream_t st);
 cudaError_t launch_pair_indforce(const double *x, const double *y, const double *z,

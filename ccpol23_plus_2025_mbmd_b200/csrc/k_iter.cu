@@ -1298,7 +1298,6 @@ constexpr int kGridSub = 16;     // sites that a row warp stages at a time
 constexpr int kGridStages = 4;  // stages of its ring, where a step's operands do not all stay
 constexpr int kGridEnt = 5;     // tensor entries that a lane has under way
 constexpr int kGridXs = 18;                    // doubles per staged site's XY (8 rows + padding)
-constexpr unsigned kGridSpins = 1u << 21;      // polls of a barrier, of about half a us each
 
 struct GridSmem {  // offsets in doubles
   int v, ring, red, part, z, rn, eim, own, src, total, ns8;
@@ -1330,15 +1329,17 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// All blocks' writes before are visible to all blocks after; false when the wait ran out.
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *ok) {
+// All blocks' writes before are visible to all blocks after; false when the wait ran out, after
+// `polls` of about half a us each.
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, unsigned polls,
+                                             int *ok) {
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     unsigned seen = 0, spins = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-    } while (seen < target && ++spins < kGridSpins);
+    } while (seen < target && ++spins < polls);
     *ok = seen >= target;
   }
   __syncthreads();
@@ -1440,7 +1441,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) k_dip_grid(IterArgs A, GridAr
   double alpha = 0.0, beta = 0.0, gamma = 0.0, chg = 0.0, ene = 0.0;
   int it = PCG ? 0 : 1;
   bool more = !PCG || A.maxit >= 1;
-  const bool started = grid_barrier(G.bar, target += gridDim.x, &ok);
+  const bool started = grid_barrier(G.bar, target += gridDim.x, G.polls, &ok);
   while (started && more) {
     const int par = it & 1;
     double *ad = G.ad + par * ad_len;
@@ -1616,7 +1617,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) k_dip_grid(IterArgs A, GridAr
         eim[3 * g + 2] = ez;
       }
     }
-    if (!grid_barrier(G.bar, target += gridDim.x, &ok)) break;
+    if (!grid_barrier(G.bar, target += gridDim.x, G.polls, &ok)) break;
     // ---- gather, two tiles of 8 sites at a time
     const int ri = (lane >> 2) & 1, cs = lane & 1, n0 = (lane >> 1) & 1, x = ri ^ cs;
     const double sg = cs == 0 && ri == 1 ? -1.0 : 1.0;
@@ -1753,7 +1754,7 @@ __global__ void __launch_bounds__(kGridThreads, 2) k_dip_grid(IterArgs A, GridAr
       }
     }
     it++;
-    if (!grid_barrier(G.bar, target += gridDim.x, &ok)) break;
+    if (!grid_barrier(G.bar, target += gridDim.x, G.polls, &ok)) break;
     if (PCG) {  // every block closes the step alike (pcg_update)
       const double *acc = G.acc + 4 * (it % 3);
       const double g1 = __ldcg(acc), d1 = __ldcg(acc + 1);
@@ -1975,11 +1976,13 @@ size_t dip_grid_scratch(const IterArgs &A) {  // doubles: counter, sums, combina
   return 16 + 2 * (size_t)((A.nrow + 7) / 8 * 8) * 4 * iter_row_tiles(A.nmax) * 4;
 }
 
-cudaError_t launch_dip_grid(const IterArgs &A, int blocks, double *scratch, cudaStream_t st) {
+cudaError_t launch_dip_grid(const IterArgs &A, int blocks, unsigned polls, double *scratch,
+                            cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(double) * dip_grid_scratch(A), st);
   if (e != cudaSuccess) return e;
   GridArgs G = {};
   G.bar = reinterpret_cast<unsigned *>(scratch);
+  G.polls = polls;
   G.acc = scratch + 4;
   G.ad = scratch + 16;
   G.ns = (A.nw + blocks - 1) / blocks;

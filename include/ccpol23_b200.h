@@ -398,6 +398,10 @@ int ccp_context_phase_ms(const ccp_context *ctx, double *ms, int n);
      "dipole_grid"   1 (default): the cooperative grid is used where it applies and no other
                      such solve is under way on the device; 0: never.  Query
                      "dipole_grid_active" tells whether the last solve used it;
+     "dipole_grid_polls" 2097152 (default): polls of a wait between the grid's blocks, of about
+                     half a microsecond each, after which it gives up: other work holds the
+                     GPU.  The evaluation is then repeated with the step kernels, which the
+                     context takes from there on, until this option or "dipole_grid" is set;
      "overlap"       1 (default): FS2 and FS3 run on low-priority side streams concurrently
                      with the Ewald and induction kernels (on a high-priority stream);
      "fs3_triples_per_block"  8 (default): FS3 triples per block when overlapping, so that
