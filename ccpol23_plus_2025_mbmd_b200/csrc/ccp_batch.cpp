@@ -18,6 +18,7 @@
 // (batch_fs3_finish).  The results equal the single-frame calls'.
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "ccp_internal.h"
@@ -38,6 +39,28 @@ int fail(int code, const std::string &msg) {
 
 const double *off(const double *p, size_t n) { return p ? p + n : nullptr; }
 double *off(double *p, size_t n) { return p ? p + n : nullptr; }
+
+// An option of all contexts that goes back to its value when the call ends.
+struct OptionForCall {
+  std::vector<std::pair<ccp_context *, int>> before;
+  const char *name = nullptr;
+  int set(const std::vector<ccp_context *> &ctx, const char *option, int value) {
+    name = option;
+    for (ccp_context *c : ctx) {
+      int v = 0;
+      int r = ccp_context_get_option(c, name, &v);
+      if (!r && v != value) {
+        r = ccp_context_set_option(c, name, value);
+        if (!r) before.push_back({c, v});
+      }
+      if (r) return r;
+    }
+    return CCP_OK;
+  }
+  ~OptionForCall() {
+    for (auto &b : before) ccp_context_set_option(b.first, name, b.second);
+  }
+};
 
 }  // namespace
 
@@ -126,16 +149,25 @@ int ccp_batch_terms_device(ccp_batch *b, unsigned terms, int nframes, const doub
     if (ncoef < 1 || pgrad_len != 2 * ncoef + 2 * 3 * 289)
       return fail(CCP_ERR_BAD_INPUT, "ccp_batch_terms_device: pgrad_len is not 2 ncoef + 1734");
   }
-  // FS3 of all frames in one launch set when they share one box length, and are too narrow for
-  // the pair form, which runs per frame
+  // FS3 of all frames in one launch set when they share one box length ...
   bool fused = b->fuse_fs3 && (terms & CCP_TERM_FS3) && nframes > 1 && x && y && z && xs && ys &&
                zs;
   for (int f = 1; fused && f < nframes; f++) fused = box[f] == box[0];
-  if (fused) fused = !ccp::fs3_pair_applies(b->ctx[0], box[0]);
   int model_s3 = 0;
   if (fused) {
     ccp_context_get_option(b->ctx[0], "fs3_available", &model_s3);
     fused = model_s3 != 0;
+  }
+  // ... and are too narrow for the pair form, which runs per frame.  The fused launch returns
+  // the parameter gradients whether or not the option "fs3_param_grad" is on; so then do the
+  // frames in its place, with the option on for this call.
+  OptionForCall grad_on;
+  if (fused && ccp::fs3_pair_applies(b->ctx[0], box[0])) {
+    fused = false;
+    if (pgrad) {
+      const int r = grad_on.set(b->ctx, "fs3_param_grad", 1);
+      if (r) return r;
+    }
   }
   unsigned rest = terms;
   if (fused) {
