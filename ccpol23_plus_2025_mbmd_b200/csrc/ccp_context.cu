@@ -104,6 +104,9 @@ struct ccp_context {
   Fs3PairBufs fpair{};
   void *d_fpair = nullptr;  // the one allocation they share
   int fpair_near = 0;      // entries of fpair.near
+  int fpair_pairs = 0, fpair_visits = 0;  // the most that was asked of ensure_fs3_pairs
+  size_t fpair_bytes = 0;
+  int opt_fs3_pair_mib = 0;  // bound on their size (MiB); 0: half of the device's free memory
   int opt_fs3_pair = 1;    // the pair form where it applies (1) or never (0)
   bool fs3_pair_active = false;
   int2 *d_pairs = nullptr;
@@ -322,20 +325,41 @@ int ensure_lists(ccp_context *c, int cap, int tri_cap, int pair_cap) {
   return CCP_OK;
 }
 
-// Buffers of FS3's pair form for at least pair_cap pairs and vcap visits per list, in one
-// allocation: a cudaMalloc costs 0.4 ms whatever its size, and a context's first evaluation
-// pays for it.  Returns false, with nothing allocated, when the device has no room: the caller
-// then takes the triple form.
+void free_fs3_pairs(ccp_context *c) {
+  if (c->d_fpair) cudaFree(c->d_fpair);
+  c->d_fpair = nullptr;
+  c->fpair = Fs3PairBufs{};
+  c->fpair_near = 0;
+  c->fpair_bytes = 0;
+}
+
+// Whether the context may take `bytes` for the pair form's buffers.  They are 0.6 MB per molecule
+// at the density of liquid water, far more than anything else here (1.2 GB at 2048 waters), and
+// the triple form does without them: without a bound from the caller they leave half of what is
+// free to others.  Up to 256 MiB the question is not worth its call to the driver (70 us): the 256
+// contexts that a batch has at most take 64 GiB so.
+bool fs3_pairs_allowed(const ccp_context *c, size_t bytes) {
+  if (c->opt_fs3_pair_mib > 0) return bytes <= (size_t)c->opt_fs3_pair_mib << 20;
+  if (bytes <= size_t(256) << 20) return true;
+  size_t avail = 0, total = 0;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= avail / 2;
+}
+
+// Buffers of FS3's pair form for at least pair_cap pairs and vcap visits per list (and as many as
+// any earlier call asked for), in one allocation: a cudaMalloc costs 0.4 ms whatever its size, and
+// a context's first evaluation pays for it.  Returns false, with nothing allocated, when they are
+// above their bound or the device has no room: the caller then takes the triple form.
 bool ensure_fs3_pairs(ccp_context *c, int pair_cap, int vcap) {
   Fs3PairBufs &B = c->fpair;
   const int near = c->nm * c->cap;
+  c->fpair_pairs = pair_cap = std::max(pair_cap, c->fpair_pairs);
+  c->fpair_visits = vcap = std::max(vcap, c->fpair_visits);
   if (B.tab && pair_cap <= B.pair_cap && vcap <= B.vcap && near <= c->fpair_near) return true;
-  pair_cap = std::max(pair_cap, B.pair_cap);
-  vcap = std::max(vcap, B.vcap);
-  if (c->d_fpair) cudaFree(c->d_fpair);
-  c->d_fpair = nullptr;
-  B = Fs3PairBufs{};
-  c->fpair_near = 0;
+  free_fs3_pairs(c);
   const size_t np = pair_cap;
   if (np * 4 * kFs3PairTab > 0xffffffffu) return false;  // a visit's table offsets are 32-bit
   size_t size = 0;
@@ -351,12 +375,14 @@ bool ensure_fs3_pairs(ccp_context *c, int pair_cap, int vcap) {
                vpart = place(np * kFs3PairWarps * sizeof(double)),
                nearb = place((size_t)near * sizeof(int)),
                head = place((size_t)c->nm * sizeof(int4));
+  if (!fs3_pairs_allowed(c, size)) return false;
   char *p = nullptr;
   if (dalloc(&p, size) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   c->d_fpair = p;
+  c->fpair_bytes = size;
   B.tab = reinterpret_cast<double2 *>(p + tab);
   B.wtab = reinterpret_cast<double2 *>(p + wtab);
   B.vis = p + vis;
@@ -957,12 +983,8 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
   // its buffers, by triples
   bool fs3_pair = (mask & T_FS3) && fs3_pair_applies(c, box);
   for (int attempt = 0; attempt < 6; attempt++) {
-    if (fs3_pair) {
-      // 17.5 pairs per molecule at the density of liquid water
-      const int pc = c->fpair.pair_cap ? c->fpair.pair_cap : 20 * nm;
-      const int vc = c->fpair.vcap ? c->fpair.vcap : 40;
-      fs3_pair = ensure_fs3_pairs(c, pc, vc);
-    }
+    // 17.5 pairs per molecule at the density of liquid water
+    if (fs3_pair) fs3_pair = ensure_fs3_pairs(c, 20 * nm, 40);
     c->fs3_pair_active = fs3_pair;
     c->launches = 0;
     c->phase_ran = 0;
@@ -1835,6 +1857,16 @@ int ccp_context_set_option(ccp_context *ctx, const char *name, int value) {
     ctx->opt_pdl = value != 0;
   } else if (n == "fs3_pair_form") {
     ctx->opt_fs3_pair = value != 0;
+  } else if (n == "fs3_pair_mib") {
+    if (value < 0) {
+      set_error("ccp_context_set_option: fs3_pair_mib must not be negative");
+      return CCP_ERR_BAD_INPUT;
+    }
+    ctx->opt_fs3_pair_mib = value;
+    if (value && ctx->fpair_bytes > (size_t)value << 20) {  // no evaluation is under way
+      CK(cudaSetDevice(ctx->device));
+      free_fs3_pairs(ctx);
+    }
   } else if (n == "fs3_fp32_passes") {
     ctx->opt_fs3_low = value != 0;
   } else if (n == "fs3_high_priority") {
@@ -1919,6 +1951,8 @@ int ccp_context_get_option(const ccp_context *ctx, const char *name, int *value)
     *value = ctx->opt_pdl;
   } else if (n == "fs3_pair_form") {
     *value = ctx->opt_fs3_pair;
+  } else if (n == "fs3_pair_mib") {
+    *value = ctx->opt_fs3_pair_mib;
   } else if (n == "fs3_pair_form_active") {
     *value = ctx->fs3_pair_active ? 1 : 0;
   } else if (n == "fs3_fp32_passes") {

@@ -417,6 +417,11 @@ int ccp_context_phase_ms(const ccp_context *ctx, double *ms, int n);
      "fs3_pair_form" 1 (default): in boxes wider than two FS3 cut-offs (12.6 A) FS3 runs by
                      molecule pairs (FP64); 0: by triples, as in smaller boxes.  Query
                      "fs3_pair_form_active" tells which ran;
+     "fs3_pair_mib"  0 (default): FS3 by pairs keeps tables of about 0.6 MB per molecule on the
+                     device (300 MB at 512 waters, per context), allocated by the first
+                     evaluation that needs them, if they are at most 256 MiB or half of
+                     the device's free memory; n > 0: if they are at most n MiB.  Where they are
+                     not allowed, or not to be had, FS3 runs by triples;
      "phase_matrix"  1 (default): the polarisable sites' phases are tabulated once per
                      evaluation as exp(i(l x + m y)) and exp(i n z) factors (when they take at
                      most 1 GiB), so a (site, k) phase is one complex product; 0: never (the

@@ -6,7 +6,7 @@ for them."""
 import numpy as np
 import pytest
 
-from ccpol23_plus_2025_mbmd_b200 import Context, Model, _lib, data_dir
+from ccpol23_plus_2025_mbmd_b200 import CcpError, Context, Model, _lib, data_dir
 from ccpol23_plus_2025_mbmd_b200.generator import water_box
 
 from conftest import rel
@@ -83,3 +83,21 @@ def test_pair_list_overflow(product, before, grad):
         for _ in range(2):
             _compare(_fs3(c, dense), ref)
             assert c.get_option("fs3_pair_form_active") == 1
+
+
+def test_memory_bound(product):
+    """Pair tables above the bound of option fs3_pair_mib: FS3 runs by triples, also where they
+    outgrow it only once a dense box's pairs are known (57 MiB for the first 2000 pairs of 100
+    molecules, some 85 for the 26 each that it has)."""
+    m = Model(data_dir("fs3"))
+    dense = water_box(m, 100, 12.65, 700, ld=28, min_oo=2.2)
+    ref = _triples(m, dense)
+    with Context(m, 100, dense.box) as c:
+        with pytest.raises(CcpError, match="negative"):
+            c.set_option("fs3_pair_mib", -1)
+        for mib, active in ((32, 0), (64, 0), (0, 1), (256, 1), (32, 0), (256, 1)):
+            c.set_option("fs3_pair_mib", mib)
+            assert c.get_option("fs3_pair_mib") == mib
+            for _ in range(2):
+                _compare(_fs3(c, dense), ref)
+                assert c.get_option("fs3_pair_form_active") == active
