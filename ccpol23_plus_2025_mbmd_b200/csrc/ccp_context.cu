@@ -984,7 +984,7 @@ int evaluate_impl(ccp_context *c, const double *px, const double *py, const doub
   bool fs3_pair = (mask & T_FS3) && fs3_pair_applies(c, box);
   for (int attempt = 0; attempt < 6; attempt++) {
     // 17.5 pairs per molecule at the density of liquid water
-    if (fs3_pair) fs3_pair = ensure_fs3_pairs(c, 20 * nm, 40);
+    if (fs3_pair) fs3_pair = fs3_pair_lists_fit(c->cap) && ensure_fs3_pairs(c, 20 * nm, 40);
     c->fs3_pair_active = fs3_pair;
     c->launches = 0;
     c->phase_ran = 0;

@@ -450,6 +450,9 @@ struct Fs3PairBufs {
   int pair_cap, vcap;
 };
 size_t fs3_visit_bytes();
+// Whether neighbour lists of this length go through the pair form's lists (up to some 7200; the
+// triple form's take 8200).
+bool fs3_pair_lists_fit(int cap);
 constexpr int kFs3PairTab = 296, kFs3PairWarps = 4;
 // tri: fs3_record_bytes() per triple, as launch_fs3_enum's.
 cudaError_t launch_fs3_pair_lists(const Fs3PairBufs &B, const double4 *comb, const int *nbr,

@@ -38,3 +38,33 @@ def test_dipole_rows_of_many_sites(product):
     assert rel(mu, mu0) <= TOL
     assert rel(F, F0) <= TOL
     assert abs(vir - vir0) <= TOL * max(abs(vir0), abs(e0))
+
+
+def test_fs3_with_the_longest_neighbour_lists(product, tmp_path):
+    """A cut-off radius that makes all of 7300 molecules neighbours: longer lists than the pair
+    form's shared memory takes, not longer than the triple form's.  FS3 runs, by triples, and gives
+    what the ordinary cut-off radius gives, which FS3 does not depend on (by pairs; both add the
+    same terms in different orders, test_gpu_fs3_pairs derives 1e-10)."""
+    nm, L = 7300, 60.23
+    for p in data_dir("fs3").iterdir():
+        t = p.read_text()
+        if p.name == "CONTROL":
+            assert t.count("9.0                 # rcut ") == 1
+            t = t.replace("9.0                 # rcut ", "53.0                # rcut ")
+        (tmp_path / p.name).write_text(t)
+    m0, m1 = Model(data_dir("fs3")), Model(tmp_path)
+    b = water_box(m0, nm, L, 6, ld=28)
+    res = []
+    for m, active in ((m1, 0), (m0, 1)):
+        f = [np.zeros_like(b.xs) for _ in range(3)]
+        c2, c3 = ([np.zeros(nm) for _ in range(3)] for _ in range(2))
+        vir = np.zeros(1)
+        with Context(m, nm, L, precision="fp64") as c:
+            e2, e3 = c.threebody_term(b.x, b.y, b.z, b.xs, b.ys, b.zs, L, *f, *c2, *c3, vir)
+            assert c.get_option("fs3_pair_form_active") == active
+        res.append((e3, np.stack(f), np.stack(c3), vir[0]))
+    (e, f, c3, vir), (e0, f0, c0, vir0) = res
+    assert abs(e - e0) <= 1e-10 * abs(e0)
+    assert rel(f, f0) <= 1e-10
+    assert rel(c3, c0) <= 1e-10
+    assert abs(vir - vir0) <= 1e-10 * abs(vir0)
