@@ -1014,7 +1014,8 @@ cudaError_t launch_pair_t(const Fs3PairBufs &B, const int *icnt, const double4 *
 size_t fs3_visit_bytes() { return sizeof(Visit); }
 // Shared memory of k_fs3_lists: a molecule's neighbours within the cut-off, at most its list.
 static size_t fs3_lists_smem(int cap) { return (size_t)cap * (3 * sizeof(double) + 2 * sizeof(int)); }
-bool fs3_pair_lists_fit(int cap) { return fs3_lists_smem(cap) <= 226 * 1024; }  // 1 KB: static arrays
+constexpr size_t kListsSmemMax = 226 * 1024;  // 1 KB for the static arrays
+bool fs3_pair_lists_fit(int cap) { return fs3_lists_smem(cap) <= kListsSmemMax; }
 static_assert(sizeof(Triple) == 64, "triple record");
 
 cudaError_t launch_fs3_pair_lists(const Fs3PairBufs &B, const double4 *comb, const int *nbr,
@@ -1024,9 +1025,9 @@ cudaError_t launch_fs3_pair_lists(const Fs3PairBufs &B, const double4 *comb, con
   k_fs3_near<<<(nm + 3) / 4, 128, 0, st>>>(comb, nbr, ncnt, cap, nm, P, B.near, B.head, B.pairv,
                                            B.pairij, B.vcnt, B.pair_cap, icnt);
   const size_t smem = fs3_lists_smem(cap);
-  if (smem > 48 * 1024) {
+  if (smem > 48 * 1024) {  // the same value from every thread: the limit is the kernel's
     cudaError_t e = cudaFuncSetAttribute(k_fs3_lists, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)kListsSmemMax);
     if (e != cudaSuccess) return e;
   }
   k_fs3_lists<<<nm + nsm * 12, 128, smem, st>>>(

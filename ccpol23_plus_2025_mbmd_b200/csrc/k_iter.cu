@@ -2082,7 +2082,10 @@ cudaError_t launch_iter_a_rows(const IterArgs &A, int nb, cudaStream_t st) {
   const auto k = zs ? (A.cu ? k_iter_a_rows<true, J, true> : k_iter_a_rows<false, J, true>)
                     : (A.cu ? k_iter_a_rows<true, J, false> : k_iter_a_rows<false, J, false>);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same value from every thread: the limit belongs to the kernel, and another context's
+    // may be launched between this call and the launch
+    cudaError_t e =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemMax);
     if (e != cudaSuccess) return e;
   }
   return launch_step(k, nb, A, st, smem);

@@ -363,10 +363,14 @@ inline int k1_of(int kl, int km, int kn) {
   return k1 < 2 ? 2 : k1;
 }
 
+// Lets the kernel take `smem` bytes.  The same value from every thread, since the limit belongs to
+// the kernel: what the gather's static arrays (3 KB) leave, enough for k_max 190 in l and m.
 template <typename F>
 cudaError_t set_smem(F kern, size_t smem) {
+  constexpr size_t kMax = 224 * 1024;
+  if (smem > kMax) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax);
   return cudaSuccess;
 }
 
