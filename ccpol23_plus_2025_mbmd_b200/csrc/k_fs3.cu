@@ -749,9 +749,11 @@ cudaError_t launch_fs3_enum(const double4 *comb, const int *nbr, const int *ncnt
                             int nm, Fs3Params P, void *rec, int tri_cap, int *icnt,
                             cudaStream_t st) {
   const size_t smem = sizeof(int) * (size_t)((cap + 1) & ~1) + 3 * sizeof(double) * (size_t)cap;
-  if (smem > 48 * 1024) {
+  if (smem > 48 * 1024) {  // the same value from every thread: the limit is the kernel's
+    constexpr size_t kMax = 227 * 1024 - 256;  // less the static arrays
+    if (smem > kMax) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_fs3_enum, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)kMax);
     if (e != cudaSuccess) return e;
   }
   k_fs3_enum<<<nm, 128, smem, st>>>(comb, nbr, ncnt, cap, nm, P, static_cast<Fs3Rec *>(rec),

@@ -388,10 +388,14 @@ inline size_t tile_smem(int k1, bool gather) {
          (gather ? sizeof(double4) * kKT + sizeof(double) * 3 * kParts * kST : 0);
 }
 
+// Lets the kernel take `smem` bytes: the same value from every thread, since the limit belongs to
+// the kernel and another context's call may come between this one and the launch.
 template <typename F>
 cudaError_t set_smem(F kern, size_t smem) {
+  constexpr size_t kMax = 227 * 1024;  // the kernels have no static arrays
+  if (smem > kMax) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax);
   return cudaSuccess;
 }
 

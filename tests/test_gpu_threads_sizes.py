@@ -39,3 +39,24 @@ def test_induction_of_two_sizes(product):
             for e, it in out:
                 assert it == ref[k][1]
                 assert abs(e - ref[k][0]) <= 1e-12 * abs(ref[k][0])
+
+
+def test_reciprocal_sums_of_two_kmax(product):
+    """The same for the sums k-vector by k-vector, at k_max 20 and 24 (70 and 82 KB)."""
+    m = Model(data_dir("fs3"))
+    b = water_box(m, 37, 10.37, 9, ld=28)
+
+    def work(k, reps):
+        res = []
+        with Context(m, b.nm, b.box, precision="fp64") as c:
+            for _ in range(reps):
+                f = [np.zeros_like(b.xs) for _ in range(3)]
+                res.append(c.kspace_ewald(b.x, b.y, b.z, b.xs, b.ys, b.zs, k, k, k, 0.4, b.box, *f,
+                                          np.zeros(1)))
+        return res
+
+    ref = {k: work(k, 1)[0] for k in (20, 24)}
+    jobs = [20, 24] * 4
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        for k, out in zip(jobs, pool.map(lambda k: work(k, 1500), jobs)):
+            assert max(abs(e - ref[k]) for e in out) <= 1e-12 * abs(ref[k])
