@@ -5,10 +5,9 @@ A step is one evaluation of the hot path of the 512-water FS2+FS3 box (L = 24.84
 seeded synthetic configuration): Ewald self/intramolecular, real and reciprocal sums,
 the induced-dipole solve with induction forces, FS2 and FS3 (SR/LR/blend).  The 2-body
 term and the integrator are outside this path.  ns/day = steps/s x 0.0005 ps x 86400 / 1000
-(dt = 0.5 fs).  Three forms are timed: FP64, the mixed-precision form, and the mixed form
-with FS3's ik/jk gradient passes in FP32.  The headline value is the fastest end to end of
-those whose relative force errors against the FP64 form (site forces, per-molecule forces,
-torques) are all <= 1e-5; every form is reported.
+(dt = 0.5 fs).  Two forms are timed: FP64 and the mixed-precision form.  The headline value is
+the faster end to end, the mixed form only if its relative force errors against the FP64 form
+(site forces, per-molecule forces, torques) are all <= 1e-5; both are reported.
 
   python bench.py [--gpus N --steps K --warmup W] [--impl reference]
 
@@ -42,12 +41,15 @@ CONFIG = "c2_512"
 # representation), as the reference computes it: ~130 FLOP + 15 MUFU-class operations
 # (6 exp, 3 sqrt, 6 reciprocals).  Counted as 145 floating-point operations.
 FS3_FLOP_PER_SITE_TRIPLE = 145.0
+# FP64 operations that FS3 by molecule pairs executes (k_fs3_pairs.cu), a DMMA counted as 512 with
+# its zero padding.  A visit of the pair kernel, three per sum: 80 DMMA (40,960), the sums with a
+# site 0 and the weights (8448 + 1728).  An energy sum: 80 DMMA (40,960), the contraction with the
+# coefficients and the edges (40,344).  A triple has one sum, two in the blend region.  Work per
+# molecule pair (tables, coefficients, forces) is not counted.
+FS3_FLOP_PER_SUM = 3 * 51136.0 + 81304.0
 # Precision forms the bench can time: context precision and options.  "mixed" is the
-# library's mixed form (PCG dipoles, FP32 FS2 terms, FP64 FS3); "mixed_fs3fp32" adds FS3's ik
-# and jk gradient passes in FP32 where FS3 runs by triples.  On the boxes timed here FS3 runs by
-# molecule pairs, in FP64 and faster, and the option has no effect.
-FORMS = {"fp64": ("fp64", {}), "mixed": ("mixed", {}),
-         "mixed_fs3fp32": ("mixed", {"fs3_fp32_passes": 1})}
+# library's mixed form (PCG dipoles, FP32 FS2 terms, FP64 FS3).
+FORMS = {"fp64": ("fp64", {}), "mixed": ("mixed", {})}
 
 
 def open_context(model, box, device, form):
@@ -615,7 +617,7 @@ def main():
 
     model, box, cfg = build_inputs(rank, args.config)
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.float32, device="cuda")  # 256 MB > L2
-    forms = ["fp64", "mixed", "mixed_fs3fp32"]
+    forms = ["fp64", "mixed"]
     results = {}
     with ClockSampler(local) as clk:
         for prec in forms:
@@ -631,6 +633,7 @@ def main():
                 r["e2e_s"] = t
                 r["h2d"], r["d2h"] = h2d, d2h
                 r["fs3_isolated_ms"] = time_fs3_isolated(ctx, box, torch)
+                r["fs3_pairs"] = ctx.get_option("fs3_pair_form_active")
                 results[prec] = r
         # whole MD steps of both forms from one short velocity-rescaled equilibration
         md = {}
@@ -695,15 +698,15 @@ def main():
     H = out[head]
     # roofline of the dominant kernel (FS3) of the headline form
     e = results[head]["energies"]
-    site_triples = (e["n_fs3_triples"] + e["n_fs3_blend"]) * 17 ** 3
-    fs3_s = H["fs3_ms"] * 1e-3
-    achieved = FS3_FLOP_PER_SITE_TRIPLE * site_triples / fs3_s / 1e12
-    # every form against the FP64 pipe: FS3 is FP64 except, in mixed_fs3fp32, two of its three
-    # gradient passes (the site-pair tables, the energy pass, the force weights and the site
-    # forces stay FP64), so the FP64 peak bounds it except for that FP32 share
-    peak = peak64
-    iso_s = results[head]["fs3_isolated_ms"] * 1e-3
-    iso = FS3_FLOP_PER_SITE_TRIPLE * site_triples / iso_s / 1e12
+    sums = e["n_fs3_triples"] + e["n_fs3_blend"]
+    site_triples = sums * 17 ** 3
+    fs3_s, iso_s = H["fs3_ms"] * 1e-3, results[head]["fs3_isolated_ms"] * 1e-3
+    ref_flop = FS3_FLOP_PER_SITE_TRIPLE * site_triples
+    # by triples (pair form off) the kernel does the reference's work, site triple by site triple
+    pairs = results[head]["fs3_pairs"]
+    flop = FS3_FLOP_PER_SUM * sums if pairs else ref_flop
+    achieved, iso = flop / fs3_s / 1e12, flop / iso_s / 1e12
+    peak = peak64  # FS3 is FP64 in both forms
     line = {
         "metric": METRIC if args.config == CONFIG else METRIC_C5,
         "value": out[head]["ns_day"], "unit": "ns/day", "n_gpus": world,
@@ -732,20 +735,27 @@ def main():
         "e2e": {"value": H["e2e_ns_day"], "unit": "ns/day",
                 "h2d_bytes_per_step": results[head]["h2d"], "d2h_bytes_per_step": results[head]["d2h"]},
         "roofline": {"bound": "fp64_pipe",
-                     "kernel": "k_fs3_pair<false> + k_fs3_energy",
+                     "kernel": "k_fs3_pair<false> + k_fs3_energy" if pairs else "k_fs3",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": "measured in this run by an FMA-chain microbenchmark "
                                     "(MEASURED_PEAKS.json has no FP32/FP64 figure)",
-                     "work": f"{FS3_FLOP_PER_SITE_TRIPLE:.0f} flop per site-triple evaluation x "
-                             f"{site_triples} site triples per launch",
+                     "work": (f"{FS3_FLOP_PER_SUM:.0f} flop per sum (three visits of the pair "
+                              f"kernel and one energy sum) x {sums} sums per evaluation, as the "
+                              "kernels execute them" if pairs else
+                              f"{FS3_FLOP_PER_SITE_TRIPLE:.0f} flop per site triple x "
+                              f"{site_triples} site triples"),
                      "duration_ms": H["fs3_ms"],
                      "note": "achieved uses the kernels' duration in the timed steps, where they "
                              "share the GPU with the Ewald/induction kernels; 'isolated' is the "
-                             "same with the three-body terms not overlapped; the work is the "
-                             "reference's, site triple by site triple, and the kernels form the "
-                             "same sums by molecule pairs with less of it",
+                             "same with the three-body terms not overlapped",
                      "isolated": {"duration_ms": iso_s * 1e3, "achieved": iso,
                                   "frac": iso / peak},
+                     # the reference's work for the same sums, which the kernels regroup into
+                     # less: a rate of results, not of the pipe
+                     "reference_work": {"flop_per_site_triple": FS3_FLOP_PER_SITE_TRIPLE,
+                                        "site_triples": site_triples,
+                                        "tflop_per_s": ref_flop / fs3_s / 1e12,
+                                        "tflop_per_s_isolated": ref_flop / iso_s / 1e12},
                      # DRAM bytes (read + write) of the pair and the energy kernel (377 and 85
                      # MB) from an ncu capture at 512 waters (31417 triples): the pairs' tables,
                      # 170 MB there, which L2 does not hold; on another box scaled by its triple
