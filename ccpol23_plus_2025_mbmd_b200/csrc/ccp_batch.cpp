@@ -15,7 +15,9 @@
 // frame after another and runs one neighbour search, one triple enumeration and one FS3
 // launch for all of them on its own stream (batch_fs3_launch), while the slots evaluate the
 // other terms; the FS3 forces, energies and parameter gradients are then added per frame
-// (batch_fs3_finish).  The results equal the single-frame calls'.
+// (batch_fs3_finish).  The results equal the single-frame calls'.  This is FS3 by triples; boxes
+// wide enough for the form by molecule pairs (12.6 A) run that per frame, fused or not: some 0.46
+// ms a frame of 256 waters, where the triples take 0.94.
 #include <string>
 #include <thread>
 #include <utility>

@@ -26,8 +26,8 @@
 // cooperative grid (k_dip_grid).  The step normally
 // runs in the row form (k_iter_a_rows, k_iter_b_rows below), which takes the
 // reciprocal sums as matrix products over the rows of the k-vector list.  k_iter_a and k_iter_b
-// take them k-vector by k-vector, from the factor tables (k_max above the row form's) or, by
-// option, from the full phase matrix [site][k].
+// take them k-vector by k-vector (k_max above the row form's, or by option), from the factor
+// tables or, where it fits in half of the L2, from the full phase matrix [site][k].
 #include <cooperative_groups.h>
 
 #include <algorithm>
